@@ -141,7 +141,7 @@ extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int pre
     // Defaults from a sweep on GB300 at 32^3x64 and 24^3x48 (gbds_op_autotune
     // refines them per lattice): FP32 recon 18 runs best with registers capped
     // for 6 blocks of 128 threads per SM, FP32 recon 12 with 64-thread blocks,
-    // FP64 (FP64-issue bound) is insensitive.
+    // FP64 has one launch shape.
     o->block = (prec == 32 && recon == 12) ? 64 : 128;
     o->nrhs = nrhs;
     o->format = format;
@@ -335,6 +335,7 @@ extern "C" int gbds_op_autotune(gbds_op op, const void *gauge, const void *psi, 
     // the tensor-core kernel
     const bool v2ok = op->nrhs == 8 || op->nrhs == 16 || op->nrhs == 32;
     if (generic(op) && !tc_eligible(op) && !v2ok) return GBDS_SUCCESS;
+    if (op->prec == 64 && !double_float(op)) return GBDS_SUCCESS;  // FP64: one kernel and launch shape
     const std::array<int, 9> key = {op->g.L[0], op->g.L[1], op->g.L[2], op->g.L[3], op->g.nd,
                                     op->prec,   op->recon,  op->nrhs,   op->format};
     {
@@ -521,7 +522,7 @@ extern "C" int gbds_op_dslash(gbds_op op, const void *gauge, const void *psi, vo
         op->prec == 32
             ? launch_dslash_f32(op->g, op->recon, gauge, psi, res, isign, cb, op->block, op->variant, s)
             : (double_float(op) ? launch_dslash_df(op->g, op->recon, gauge, psi, res, isign, cb, op->block, op->variant, s)
-                                : launch_dslash_f64(op->g, op->recon, gauge, psi, res, isign, cb, op->block, op->variant, s));
+                                : launch_dslash_f64(op->g, op->recon, gauge, psi, res, isign, cb, s));
     return e == cudaSuccess ? GBDS_SUCCESS : cuda_error(e, "dslash");
 }
 
@@ -726,7 +727,7 @@ void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, i
         if (e == cudaSuccess) e = launch_pack_spinor(g, prec, dpsi, nullptr, 0, cb, c.d_psi, s);
         if (e == cudaSuccess)
             e = prec == 32 ? launch_dslash_f32(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s)
-                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s);
+                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, s);
         if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, nullptr, 0, target, dres, s);
         cudaError_t e2 = cudaStreamSynchronize(s);
         if (e == cudaSuccess) e = e2;
@@ -750,7 +751,7 @@ void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, i
         if (e == cudaSuccess) e = launch_pack_spinor(g, prec, c.d_psi_packed, nullptr, cb * g.Vh, cb, c.d_psi, s);
         if (e == cudaSuccess)
             e = prec == 32 ? launch_dslash_f32(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s)
-                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s);
+                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, s);
         if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, nullptr, target * g.Vh, target, c.d_res_packed, s);
         char *dst = static_cast<char *>(res) + (size_t)target * g.Vh * spinor;
         if (e == cudaSuccess) e = cudaMemcpyAsync(dst, c.d_res_packed, (size_t)g.Vh * spinor, cudaMemcpyDeviceToHost, s);
@@ -762,7 +763,7 @@ void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, i
         if (e == cudaSuccess) e = launch_pack_spinor(g, prec, c.d_psi_packed, table, 0, cb, c.d_psi, s);
         if (e == cudaSuccess)
             e = prec == 32 ? launch_dslash_f32(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s)
-                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s);
+                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, s);
         if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, table, 0, target, c.d_res_packed, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(res, c.d_res_packed, (size_t)g.V * spinor, cudaMemcpyDeviceToHost, s);
     }

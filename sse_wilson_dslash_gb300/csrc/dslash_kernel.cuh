@@ -470,10 +470,9 @@ __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks) d
     Field<T>::store_spinor(a.res, a.g.stride, h, acc);
 }
 
-// Register-cap variants: index -> MINB (see Bounds).  FP32 and FP64 differ.
+// Register-cap variants: index -> MINB (see Bounds).
 template <typename T> struct Variants;
 template <> struct Variants<float> { static constexpr int n = 5; static constexpr int minb[5] = {0, 6, 7, 8, 10}; };
-template <> struct Variants<double> { static constexpr int n = 3; static constexpr int minb[3] = {0, 3, 4}; };
 // double-float at 32^3x64: 1.28 ms uncapped, 0.86 ms at 3 and 0.74 ms at 4
 // CTAs of 128 threads per SM; 5 and 6 spill 1.2-1.9 KB and lose
 template <> struct Variants<dfloat> { static constexpr int n = 3; static constexpr int minb[3] = {0, 3, 4}; };
@@ -588,7 +587,6 @@ __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks)
 
 template <typename T> struct XpayMinb;
 template <> struct XpayMinb<float> { static constexpr int r18 = 6, r12 = 6; };
-template <> struct XpayMinb<double> { static constexpr int r18 = 0, r12 = 0; };
 template <> struct XpayMinb<dfloat> { static constexpr int r18 = 4, r12 = 4; };
 
 // Grid blocks of an xpay launch (the size `partials` must have).

@@ -38,8 +38,10 @@ void count_launch(int n = 1);
 // (0 = uncapped; see Variants<T> in dslash_kernel.cuh).
 cudaError_t launch_dslash_f32(const Geom &g, int recon, const void *gauge, const void *psi,
                               void *res, int isign, int cb, int block, int variant, cudaStream_t stream);
+// FP64: one kernel and launch shape (dslash_f64.cu)
 cudaError_t launch_dslash_f64(const Geom &g, int recon, const void *gauge, const void *psi,
-                              void *res, int isign, int cb, int block, int variant, cudaStream_t stream);
+                              void *res, int isign, int cb, cudaStream_t stream);
+// variant indices the tuning calls accept (FP64: three, all the same kernel)
 int dslash_variants(int prec);
 
 // res = x + coef * Dslash(psi) (4D; res and x on checkerboard 1-cb); if
@@ -47,8 +49,9 @@ int dslash_variants(int prec);
 // (there are (Vh + 127) / 128 blocks).
 cudaError_t launch_dslash_xpay_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
                                    float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream);
-cudaError_t launch_dslash_xpay_f64(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
-                                   double coef, void *res, double *partials, int isign, int cb, cudaStream_t stream);
+// (18-real links)
+cudaError_t launch_dslash_xpay_f64(const Geom &g, const void *gauge, const void *psi, const void *x, double coef,
+                                   void *res, double *partials, int isign, int cb, cudaStream_t stream);
 
 // Double-float (dslash_df.cu, dfloat.cuh): FP64 fields stored as (hi, lo)
 // FP32 pairs, 16 bytes a complex as in FP64, computed on the FP32 pipes.

@@ -397,14 +397,14 @@ template <typename T>
 cudaError_t dslash(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign, int cb,
                    int block, int variant, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) return launch_dslash_f32(g, recon, gauge, psi, res, isign, cb, block, variant, st);
-    else return launch_dslash_f64(g, recon, gauge, psi, res, isign, cb, block, variant, st);
+    else return launch_dslash_f64(g, recon, gauge, psi, res, isign, cb, st);
 }
 
 template <typename T>
 cudaError_t dslash_xpay(const Geom &g, int recon, const void *gauge, const void *psi, const void *x, T coef, void *res,
                         double *partials, int isign, int cb, cudaStream_t st) {
     if constexpr (sizeof(T) == 4) return launch_dslash_xpay_f32(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st);
-    else return launch_dslash_xpay_f64(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st);
+    else return launch_dslash_xpay_f64(g, gauge, psi, x, coef, res, partials, isign, cb, st);
 }
 
 cudaError_t finish_on(gbds_solver s, int mode, cudaStream_t st) {
