@@ -11,4 +11,10 @@ cudaError_t launch_dslash_xpay_f32(const Geom &g, int recon, const void *gauge, 
                                    float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream) {
     return launch_dslash_xpay_t<float>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, stream);
 }
+cudaError_t launch_dslash_cg_update_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
+                                        float coef, const double *alpha, void *r, double *partials, int isign, int cb,
+                                        cudaStream_t stream) {
+    return launch_dslash_xpay_t<float, true>(g, recon, gauge, psi, x, coef, nullptr, partials, isign, cb, stream,
+                                             {static_cast<float4 *>(r), alpha});
+}
 }  // namespace gbds

@@ -275,12 +275,14 @@ __device__ __forceinline__ void fx_plain_dir(const DslashArgs<double> &a, int c,
     fx_plain_hop<MU, -ISIGN, true, ND, RECON>(a, c, n.b[MU], n.b[MU], 1 - a.pt, acc);
 }
 
-// res = Dslash psi, or (XPAY) x + coef Dslash psi with partials[block] = the
-// block's sum of |res|^2 where partials != nullptr.  GROUPS groups of three
+// res = Dslash psi, or (EPI 1) x + coef Dslash psi with partials[block] = the
+// block's sum of |res|^2 where partials != nullptr, or (EPI 2) the CG's update
+// r -= alpha (x + coef Dslash psi) in place of the store, with |r|^2.  GROUPS groups of three
 // warps a CTA: 1, or 4 where partials of 128-site blocks are wanted.
-template <int ND, int RECON, int ISIGN, bool XPAY, int GROUPS>
+template <int ND, int RECON, int ISIGN, int EPI, int GROUPS>
 __global__ void __launch_bounds__(96 * GROUPS, GROUPS == 1 ? 7 : 2)
-    dslash_fx_kernel(const DslashArgs<double> a, const double2 *__restrict__ x, double coef, double *partials) {
+    dslash_fx_kernel(const DslashArgs<double> a, const double2 *__restrict__ x, double coef, const CgUpdate<double> upd,
+                     double *partials) {
     __shared__ FxShared<GROUPS> sm;
     pdl_allow_next();
     const int warp = threadIdx.x >> 5;
@@ -318,16 +320,22 @@ __global__ void __launch_bounds__(96 * GROUPS, GROUPS == 1 ? 7 : 2)
 #pragma unroll
         for (int sp = 0; sp < 4; sp++) {
             const size_t i = (size_t)(sp * 3 + th.c) * a.g.stride + h;
-            if constexpr (XPAY) {
+            if constexpr (EPI) {
                 const double2 xv = __ldg(x + i);
                 r[sp] = {fma(coef, r[sp].r, xv.x), fma(coef, r[sp].i, xv.y)};
+                if constexpr (EPI == 2) {
+                    const double al = -*upd.alpha;
+                    const double2 ro = upd.r[i];
+                    r[sp] = {fma(al, r[sp].r, ro.x), fma(al, r[sp].i, ro.y)};
+                }
                 nrm = fma(r[sp].r, r[sp].r, nrm);
                 nrm = fma(r[sp].i, r[sp].i, nrm);
             }
-            __stcs(a.res + i, make_double2(r[sp].r, r[sp].i));
+            if constexpr (EPI == 2) upd.r[i] = make_double2(r[sp].r, r[sp].i);
+            else __stcs(a.res + i, make_double2(r[sp].r, r[sp].i));
         }
     }
-    if constexpr (XPAY) {
+    if constexpr (EPI) {
         if (partials) block_sum_to<double>(partials, nrm);
     }
 }
@@ -343,13 +351,13 @@ DslashArgs<double> f64_args(const Geom &g, int recon, const void *gauge, const v
     return a;
 }
 
-template <int ND, int RECON, bool XPAY, int GROUPS>
+template <int ND, int RECON, int EPI, int GROUPS>
 cudaError_t launch_fx(const DslashArgs<double> &a, int isign, const double2 *x, double coef, double *partials,
-                      cudaStream_t st) {
+                      cudaStream_t st, const CgUpdate<double> &upd = {}) {
     const dim3 grid((a.g.Vh + kFxSites * GROUPS - 1) / (kFxSites * GROUPS));
     const int threads = 96 * GROUPS;
-    if (isign > 0) launch_pdl(dslash_fx_kernel<ND, RECON, 1, XPAY, GROUPS>, grid, threads, st, a, x, coef, partials);
-    else launch_pdl(dslash_fx_kernel<ND, RECON, -1, XPAY, GROUPS>, grid, threads, st, a, x, coef, partials);
+    if (isign > 0) launch_pdl(dslash_fx_kernel<ND, RECON, 1, EPI, GROUPS>, grid, threads, st, a, x, coef, upd, partials);
+    else launch_pdl(dslash_fx_kernel<ND, RECON, -1, EPI, GROUPS>, grid, threads, st, a, x, coef, upd, partials);
     count_launch();
     return cudaGetLastError();
 }
@@ -362,10 +370,10 @@ cudaError_t launch_dslash_f64(const Geom &g, int recon, const void *gauge, const
                               cudaStream_t stream) {
     const DslashArgs<double> a = f64_args(g, recon, gauge, psi, res, cb);
     if (g.nd == 4)
-        return recon == 18 ? launch_fx<4, 18, false, 1>(a, isign, nullptr, 0.0, nullptr, stream)
-                           : launch_fx<4, 12, false, 1>(a, isign, nullptr, 0.0, nullptr, stream);
-    return recon == 18 ? launch_fx<3, 18, false, 1>(a, isign, nullptr, 0.0, nullptr, stream)
-                       : launch_fx<3, 12, false, 1>(a, isign, nullptr, 0.0, nullptr, stream);
+        return recon == 18 ? launch_fx<4, 18, 0, 1>(a, isign, nullptr, 0.0, nullptr, stream)
+                           : launch_fx<4, 12, 0, 1>(a, isign, nullptr, 0.0, nullptr, stream);
+    return recon == 18 ? launch_fx<3, 18, 0, 1>(a, isign, nullptr, 0.0, nullptr, stream)
+                       : launch_fx<3, 12, 0, 1>(a, isign, nullptr, 0.0, nullptr, stream);
 }
 
 // 4D, 18-real links (the solvers' FP64 links)
@@ -373,8 +381,15 @@ cudaError_t launch_dslash_xpay_f64(const Geom &g, const void *gauge, const void 
                                    void *res, double *partials, int isign, int cb, cudaStream_t stream) {
     const DslashArgs<double> a = f64_args(g, 18, gauge, psi, res, cb);
     const double2 *xv = static_cast<const double2 *>(x);
-    return partials ? launch_fx<4, 18, true, 4>(a, isign, xv, coef, partials, stream)
-                    : launch_fx<4, 18, true, 1>(a, isign, xv, coef, nullptr, stream);
+    return partials ? launch_fx<4, 18, 1, 4>(a, isign, xv, coef, partials, stream)
+                    : launch_fx<4, 18, 1, 1>(a, isign, xv, coef, nullptr, stream);
+}
+
+cudaError_t launch_dslash_cg_update_f64(const Geom &g, const void *gauge, const void *psi, const void *x, double coef,
+                                        const double *alpha, void *r, double *partials, int isign, int cb,
+                                        cudaStream_t stream) {
+    return launch_fx<4, 18, 2, 4>(f64_args(g, 18, gauge, psi, nullptr, cb), isign, static_cast<const double2 *>(x), coef,
+                                  partials, stream, {static_cast<double2 *>(r), alpha});
 }
 
 }  // namespace gbds

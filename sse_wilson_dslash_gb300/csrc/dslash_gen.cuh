@@ -230,6 +230,7 @@ struct GenArgs {
     // per-(block, rhs) |r|^2 partials
     const RhsCgScalars *rsc;
     float4 *rvec;
+    const double *alpha;  // the same for nrhs 1 (16-bit storage, rvec an FP32 field)
 };
 
 // NRHS > 0: compile-time count; NRHS == 0: a.nrhs at run time.
@@ -1066,7 +1067,9 @@ __global__ void __launch_bounds__(128, G5Smem<FMT, NRHS>::MINB) dslash_gen5_kern
 
 // One thread per (site, rhs); 4D.  EPI = 1 adds the xpay epilogue
 // (res = x + coef * D psi) with one |res|^2 partial per block; EPI = 2 the
-// same with one partial per block and rhs (NRHS 2..32, 128-thread blocks).
+// same with one partial per block and rhs (NRHS 2..32, 128-thread blocks);
+// EPI = 3 (NRHS 1) the CG update r -= alpha (x + coef * D psi) on the FP32 field
+// rvec instead of the store, with |r|^2.
 template <int FMT, int RECON, int ISIGN, int NRHS, int EPI, int LFMT = 0>
 __global__ void __launch_bounds__(128, 6) dslash_gen_kernel(const GenArgs a) {
     pdl_allow_next();
@@ -1098,13 +1101,29 @@ __global__ void __launch_bounds__(128, 6) dslash_gen_kernel(const GenArgs a) {
                 for (int c = 0; c < 3; c++) {
                     acc[s][c].r = fmaf(a.coef, acc[s][c].r, xv[s][c].r);
                     acc[s][c].i = fmaf(a.coef, acc[s][c].i, xv[s][c].i);
-                    nrm = fmaf(acc[s][c].r, acc[s][c].r, nrm);
-                    nrm = fmaf(acc[s][c].i, acc[s][c].i, nrm);
+                    if constexpr (EPI != 3) {
+                        nrm = fmaf(acc[s][c].r, acc[s][c].r, nrm);
+                        nrm = fmaf(acc[s][c].i, acc[s][c].i, nrm);
+                    }
                 }
         }
-        Sio<FMT>::store(a.res, a.cs, i, acc);
+        if constexpr (EPI == 3) {
+            const float al = -(float)*a.alpha;
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                const cx<float> u = acc[(2 * k) / 3][(2 * k) % 3], v = acc[(2 * k + 1) / 3][(2 * k + 1) % 3];
+                float4 *rp = a.rvec + (size_t)k * a.g.stride + h;
+                const float4 ro = *rp;
+                const float4 rn = make_float4(fmaf(al, u.r, ro.x), fmaf(al, u.i, ro.y), fmaf(al, v.r, ro.z),
+                                              fmaf(al, v.i, ro.w));
+                *rp = rn;
+                nrm += rn.x * rn.x + rn.y * rn.y + rn.z * rn.z + rn.w * rn.w;
+            }
+        } else {
+            Sio<FMT>::store(a.res, a.cs, i, acc);
+        }
     }
-    if constexpr (EPI == 1) {
+    if constexpr (EPI == 1 || EPI == 3) {
         if (a.partials) block_sum_to<float>(a.partials, nrm);
     } else if constexpr (EPI == 2) {
         if (a.partials) block_sum_rhs<NRHS>(a.partials, nrm);

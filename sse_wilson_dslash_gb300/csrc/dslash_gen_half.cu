@@ -10,9 +10,10 @@ cudaError_t launch_gen_half(int fmt, const Geom &g, int recon, int nrhs, const v
     return launch_gen_t<kFmtF16N>(g, recon, nrhs, gauge, psi, res, isign, cb, x, coef, partials, st, variant);
 }
 cudaError_t launch_gen_h16(int fmt, const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign,
-                           int cb, const void *x, float coef, double *partials, cudaStream_t st) {
-    if (fmt == kFmtBF16) return launch_gen_h16_t<kFmtBF16>(g, recon, gauge, psi, res, isign, cb, x, coef, partials, st);
-    return launch_gen_h16_t<kFmtF16N>(g, recon, gauge, psi, res, isign, cb, x, coef, partials, st);
+                           int cb, const void *x, float coef, double *partials, cudaStream_t st, void *r, const double *alpha) {
+    if (fmt == kFmtBF16)
+        return launch_gen_h16_t<kFmtBF16>(g, recon, gauge, psi, res, isign, cb, x, coef, partials, st, r, alpha);
+    return launch_gen_h16_t<kFmtF16N>(g, recon, gauge, psi, res, isign, cb, x, coef, partials, st, r, alpha);
 }
 
 // FP32 internal links -> FP16 internal links, element by element (same

@@ -61,7 +61,7 @@ void launch_gen_nrhs(const GenArgs &a, int nrhs, dim3 grid, cudaStream_t st) {
 // nrhs 1 with FP16 links (the 16-bit inner solver's operator)
 template <int FMT>
 cudaError_t launch_gen_h16_t(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign, int cb,
-                             const void *x, float coef, double *partials, cudaStream_t st) {
+                             const void *x, float coef, double *partials, cudaStream_t st, void *r, const double *alpha) {
     GenArgs a;
     a.g = g;
     a.psi = static_cast<const char *>(psi);
@@ -76,7 +76,12 @@ cudaError_t launch_gen_h16_t(const Geom &g, int recon, const void *gauge, const 
     a.partials = partials;
     const dim3 grid((unsigned)((g.Vh + 127) / 128));
 #define GBDS_H(R, S, E) launch_pdl(dslash_gen_kernel<FMT, R, S, 1, E, 1>, grid, 128, st, a)
-    if (x) {
+    a.rvec = static_cast<float4 *>(r);
+    a.alpha = alpha;
+    if (r) {
+        if (recon == 18) { if (isign > 0) GBDS_H(18, 1, 3); else GBDS_H(18, -1, 3); }
+        else             { if (isign > 0) GBDS_H(12, 1, 3); else GBDS_H(12, -1, 3); }
+    } else if (x) {
         if (recon == 18) { if (isign > 0) GBDS_H(18, 1, 1); else GBDS_H(18, -1, 1); }
         else             { if (isign > 0) GBDS_H(12, 1, 1); else GBDS_H(12, -1, 1); }
     } else {

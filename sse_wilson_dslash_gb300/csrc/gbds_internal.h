@@ -49,7 +49,15 @@ int dslash_variants(int prec);
 // (there are (Vh + 127) / 128 blocks).
 cudaError_t launch_dslash_xpay_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
                                    float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream);
+// r -= alpha (x + coef * Dslash(psi)), alpha read on the device, with |r|^2 in
+// the partials (as above)
+cudaError_t launch_dslash_cg_update_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
+                                        float coef, const double *alpha, void *r, double *partials, int isign, int cb,
+                                        cudaStream_t stream);
 // (18-real links)
+cudaError_t launch_dslash_cg_update_f64(const Geom &g, const void *gauge, const void *psi, const void *x, double coef,
+                                        const double *alpha, void *r, double *partials, int isign, int cb,
+                                        cudaStream_t stream);
 cudaError_t launch_dslash_xpay_f64(const Geom &g, const void *gauge, const void *psi, const void *x, double coef,
                                    void *res, double *partials, int isign, int cb, cudaStream_t stream);
 
@@ -117,11 +125,13 @@ cudaError_t launch_gen_tc(int fmt, const Geom &g, int recon, int nrhs, const voi
 // The tensor-core kernel's bounded mbarrier wait on a barrier nothing
 // completes; flag = 1 when the wait gave up.
 cudaError_t launch_tc_wait_selftest(int polls, int *flag, cudaStream_t st);
-// nrhs 1, 16-bit spinors (fmt 1 / 2) with FP16 links: gauge is the FP32
+// nrhs 1, 16-bit spinors (fmt 1 / 2) with FP16 links (r, alpha set: the CG
+// update r -= alpha (x + coef D psi) on the FP32 field r instead of the store): gauge is the FP32
 // internal gauge converted by convert_links_f16 (recon * 2 bytes per link
 // per site-stride).
 cudaError_t launch_gen_h16(int fmt, const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign,
-                           int cb, const void *x, float coef, double *partials, cudaStream_t st);
+                           int cb, const void *x, float coef, double *partials, cudaStream_t st, void *r = nullptr,
+                           const double *alpha = nullptr);
 cudaError_t convert_links_f16(const void *gauge32, void *gauge16, size_t nfloats, cudaStream_t st);
 
 // Sizes in bytes of the internal fields.

@@ -14,7 +14,7 @@
 //                  instead of four).  The normal-equation solve keeps
 //                  r = c - A x in FP64.
 //   inner_prec 16 / 17: the same with the CG's direction p and the operator's
-//                  intermediates (M p, A p, D_oe p) stored as half with a
+//                  intermediates (M p, D_oe p) stored as half with a
 //                  per-site norm (16) or bfloat16 (17), FP16 links, FP32
 //                  arithmetic; the CG's solution and residual stay FP32.
 // The reference library provides only D; a caller such as Chroma builds M and
@@ -59,42 +59,22 @@ __device__ __forceinline__ double2 axpy_v(double a, double2 x, double2 y) {
 __device__ __forceinline__ float norm_v(float4 v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
 __device__ __forceinline__ double norm_v(double2 v) { return v.x * v.x + v.y * v.y; }
 
-// x += alpha p;  r -= alpha Ap;  partial |r|^2
+// x += alpha p;  p = r + beta p  (r -= alpha A p is M^+'s second launch's, the
+// update epilogue of the Dslash kernels)
 template <typename T>
-__global__ void __launch_bounds__(kThreads) cg_update(SV<T> *x, SV<T> *r, const SV<T> *__restrict__ p,
-                                                     const SV<T> *__restrict__ Ap, const Scalars *sc, int Vh, int stride,
-                                                     double *partials) {
-    pdl_allow_next();
-    pdl_wait_prev();
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    T nrm = 0;
-    if (h < Vh) {
-        const T a = (T)sc->alpha;
-#pragma unroll
-        for (int k = 0; k < nvec<T>(); k++) {
-            const size_t i = (size_t)k * stride + h;
-            x[i] = axpy_v(a, p[i], x[i]);
-            const SV<T> rn = axpy_v(-a, Ap[i], r[i]);
-            r[i] = rn;
-            nrm += norm_v(rn);
-        }
-    }
-    block_sum_to<T>(partials, nrm);
-}
-
-// p = r + beta p
-template <typename T>
-__global__ void __launch_bounds__(kThreads) cg_xpay(const SV<T> *__restrict__ r, SV<T> *p, const Scalars *sc, int Vh,
-                                                   int stride) {
+__global__ void __launch_bounds__(kThreads) cg_xpay(const SV<T> *__restrict__ r, SV<T> *x, SV<T> *p, const Scalars *sc,
+                                                   int Vh, int stride) {
     pdl_allow_next();
     pdl_wait_prev();
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= Vh) return;
-    const T b = (T)sc->beta;
+    const T a = (T)sc->alpha, b = (T)sc->beta;
 #pragma unroll
     for (int k = 0; k < nvec<T>(); k++) {
         const size_t i = (size_t)k * stride + h;
-        p[i] = axpy_v(b, p[i], r[i]);
+        const SV<T> pv = p[i];
+        x[i] = axpy_v(a, pv, x[i]);
+        p[i] = axpy_v(b, pv, r[i]);
     }
 }
 
@@ -246,45 +226,22 @@ __device__ __forceinline__ float4 pair(const cx<float> (&s)[4][3], int k) {
     return make_float4(a.r, a.i, b.r, b.i);
 }
 
-// x += alpha p;  r -= alpha Ap;  partial |r|^2   (p, Ap 16-bit)
+// x += alpha p;  p = r + beta p   (p 16-bit)
 template <int FMT>
-__global__ void __launch_bounds__(kThreads) cg_update_h(float4 *x, float4 *r, const char *p, const char *Ap,
-                                                       const Scalars *sc, int Vh, int stride, double *partials) {
-    pdl_allow_next();
-    pdl_wait_prev();
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    float nrm = 0.f;
-    if (h < Vh) {
-        const float a = (float)sc->alpha;
-        cx<float> ps[4][3], aps[4][3];
-        Sio<FMT>::load(p, stride, h, ps);
-        Sio<FMT>::load(Ap, stride, h, aps);
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            const size_t i = (size_t)k * stride + h;
-            x[i] = axpy_v(a, pair(ps, k), x[i]);
-            const float4 rn = axpy_v(-a, pair(aps, k), r[i]);
-            r[i] = rn;
-            nrm += norm_v(rn);
-        }
-    }
-    block_sum_to<float>(partials, nrm);
-}
-
-// p = r + beta p   (p 16-bit)
-template <int FMT>
-__global__ void __launch_bounds__(kThreads) cg_xpay_h(const float4 *__restrict__ r, char *p, const Scalars *sc, int Vh,
-                                                     int stride) {
+__global__ void __launch_bounds__(kThreads) cg_xpay_h(const float4 *__restrict__ r, float4 *x, char *p, const Scalars *sc,
+                                                     int Vh, int stride) {
     pdl_allow_next();
     pdl_wait_prev();
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= Vh) return;
-    const float b = (float)sc->beta;
+    const float a = (float)sc->alpha, b = (float)sc->beta;
     cx<float> ps[4][3];
     Sio<FMT>::load(p, stride, h, ps);
 #pragma unroll
     for (int k = 0; k < 6; k++) {
-        const float4 rv = r[(size_t)k * stride + h];
+        const size_t i = (size_t)k * stride + h;
+        const float4 rv = r[i];
+        x[i] = axpy_v(a, pair(ps, k), x[i]);
         cx<float> &u = ps[(2 * k) / 3][(2 * k) % 3];
         cx<float> &v = ps[(2 * k + 1) / 3][(2 * k + 1) % 3];
         u = {fmaf(b, u.r, rv.x), fmaf(b, u.i, rv.y)};
@@ -379,9 +336,9 @@ struct gbds_solver_s {
     void *b64 = nullptr, *c64 = nullptr, *x64 = nullptr, *r64 = nullptr, *p64 = nullptr, *Ap64 = nullptr,
          *Mp64 = nullptr, *t64 = nullptr;
     // FP32 inner fields
-    void *e32 = nullptr, *r32 = nullptr, *p32 = nullptr, *Ap32 = nullptr, *Mp32 = nullptr, *t32 = nullptr;
+    void *e32 = nullptr, *r32 = nullptr, *p32 = nullptr, *Mp32 = nullptr, *t32 = nullptr;
     // 16-bit inner fields and FP16 links (inner_prec 16 / 17)
-    void *p16 = nullptr, *Ap16 = nullptr, *Mp16 = nullptr, *t16 = nullptr, *gauge16 = nullptr;
+    void *p16 = nullptr, *Mp16 = nullptr, *t16 = nullptr, *gauge16 = nullptr;
     int fmt16 = 0;
     double *partials = nullptr;
     Scalars *sc = nullptr;    // device
@@ -395,8 +352,9 @@ namespace {
 // instantiated once, in dslash_f32.cu / dslash_f64.cu).
 template <typename T>
 cudaError_t dslash(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign, int cb,
-                   int block, int variant, cudaStream_t st) {
-    if constexpr (sizeof(T) == 4) return launch_dslash_f32(g, recon, gauge, psi, res, isign, cb, block, variant, st);
+                   cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) return launch_dslash_f32(g, recon, gauge, psi, res, isign, cb, recon == 12 ? 64 : 128,
+                                                           recon == 18 ? 1 : 0, st);
     else return launch_dslash_f64(g, recon, gauge, psi, res, isign, cb, st);
 }
 
@@ -419,11 +377,23 @@ cudaError_t apply_M(gbds_solver s, const void *gauge, int recon, const void *in,
                     double *partials, cudaStream_t st) {
     const Geom &g = s->g;
     const double k2 = s->prm.kappa * s->prm.kappa;
-    const int variant = (sizeof(T) == 4 && recon == 18) ? 1 : 0;
-    const int block = (sizeof(T) == 4 && recon == 12) ? 64 : 128;
-    cudaError_t e = dslash<T>(g, recon, gauge, in, tmp, isign, 0, block, variant, st);
+    cudaError_t e = dslash<T>(g, recon, gauge, in, tmp, isign, 0, st);
     if (e != cudaSuccess) return e;
     return dslash_xpay<T>(g, recon, gauge, tmp, in, (T)(-k2), out, partials, isign, 1, st);
+}
+
+// r -= alpha M^+ in, |r|^2 in the partials: M^+'s second launch updates r in
+// place of storing M^+ in
+template <typename T>
+cudaError_t apply_Mdag_update(gbds_solver s, const void *gauge, int recon, const void *in, void *tmp, void *r,
+                              cudaStream_t st) {
+    const Geom &g = s->g;
+    const double k2 = s->prm.kappa * s->prm.kappa;
+    cudaError_t e = dslash<T>(g, recon, gauge, in, tmp, -1, 0, st);
+    if (e != cudaSuccess) return e;
+    if constexpr (sizeof(T) == 4)
+        return launch_dslash_cg_update_f32(g, recon, gauge, tmp, in, (float)(-k2), &s->sc->alpha, r, s->partials, -1, 1, st);
+    else return launch_dslash_cg_update_f64(g, gauge, tmp, in, -k2, &s->sc->alpha, r, s->partials, -1, 1, st);
 }
 
 // The outer residual's operator in double-float (outer_double_float): out
@@ -489,7 +459,7 @@ cudaError_t read_scalars(gbds_solver s, cudaStream_t st) {
 // CG on A = M^+ M with x, r, p prepared (x = 0, r = p = rhs, sc->rr = |rhs|^2).
 // Stops when rr <= target_rr or after max_iter iterations.
 template <typename T>
-cudaError_t cg(gbds_solver s, const void *gauge, int recon, void *x, void *r, void *p, void *Ap, void *Mp, void *t,
+cudaError_t cg(gbds_solver s, const void *gauge, int recon, void *x, void *r, void *p, void *Mp, void *t,
                double target_rr, int max_iter, int *iters, cudaStream_t st) {
     const Geom &g = s->g;
     const int nb = blocks(g);
@@ -501,18 +471,11 @@ cudaError_t cg(gbds_solver s, const void *gauge, int recon, void *x, void *r, vo
     while (k < max_iter) {
         e = apply_M<T>(s, gauge, recon, p, t, Mp, +1, s->partials, st);
         if (e == cudaSuccess) e = finish_on(s, kAlpha, st);
-        if (e == cudaSuccess) e = apply_M<T>(s, gauge, recon, Mp, t, Ap, -1, nullptr, st);
-        if (e == cudaSuccess) {
-            launch_pdl(cg_update<T>, dim3(nb), kThreads, st, static_cast<SV<T> *>(x), static_cast<SV<T> *>(r),
-                       static_cast<const SV<T> *>(p), static_cast<const SV<T> *>(Ap), (const Scalars *)s->sc, g.Vh,
-                       g.stride, s->partials);
-            count_launch();
-            e = cudaGetLastError();
-        }
+        if (e == cudaSuccess) e = apply_Mdag_update<T>(s, gauge, recon, Mp, t, r, st);
         if (e == cudaSuccess) e = finish_on(s, kBeta, st);
         if (e == cudaSuccess) {
-            launch_pdl(cg_xpay<T>, dim3(nb), kThreads, st, static_cast<const SV<T> *>(r), static_cast<SV<T> *>(p),
-                       (const Scalars *)s->sc, g.Vh, g.stride);
+            launch_pdl(cg_xpay<T>, dim3(nb), kThreads, st, static_cast<const SV<T> *>(r), static_cast<SV<T> *>(x),
+                       static_cast<SV<T> *>(p), (const Scalars *)s->sc, g.Vh, g.stride);
             count_launch();
             e = cudaGetLastError();
         }
@@ -538,6 +501,15 @@ cudaError_t apply_M_h(gbds_solver s, const void *in, void *tmp, void *out, int i
     return launch_gen_h16(s->fmt16, g, s->prm.inner_recon, s->gauge16, tmp, out, isign, 1, in, -k2, partials, st);
 }
 
+cudaError_t apply_Mdag_update_h(gbds_solver s, const void *in, void *tmp, void *r, cudaStream_t st) {
+    const Geom &g = s->g;
+    const float k2 = (float)(s->prm.kappa * s->prm.kappa);
+    cudaError_t e = launch_gen_h16(s->fmt16, g, s->prm.inner_recon, s->gauge16, in, tmp, -1, 0, nullptr, 0.f, nullptr, st);
+    if (e != cudaSuccess) return e;
+    return launch_gen_h16(s->fmt16, g, s->prm.inner_recon, s->gauge16, tmp, nullptr, -1, 1, in, -k2, s->partials, st, r,
+                          &s->sc->alpha);
+}
+
 template <int FMT>
 cudaError_t cg_h(gbds_solver s, double target_rr, int max_iter, int *iters, cudaStream_t st) {
     const Geom &g = s->g;
@@ -549,18 +521,11 @@ cudaError_t cg_h(gbds_solver s, double target_rr, int max_iter, int *iters, cuda
     while (k < max_iter) {
         e = apply_M_h(s, s->p16, s->t16, s->Mp16, +1, s->partials, st);
         if (e == cudaSuccess) e = finish_on(s, kAlpha, st);
-        if (e == cudaSuccess) e = apply_M_h(s, s->Mp16, s->t16, s->Ap16, -1, nullptr, st);
-        if (e == cudaSuccess) {
-            launch_pdl(cg_update_h<FMT>, dim3(nb), kThreads, st, static_cast<float4 *>(s->e32),
-                       static_cast<float4 *>(s->r32), static_cast<const char *>(s->p16),
-                       static_cast<const char *>(s->Ap16), (const Scalars *)s->sc, g.Vh, g.stride, s->partials);
-            count_launch();
-            e = cudaGetLastError();
-        }
+        if (e == cudaSuccess) e = apply_Mdag_update_h(s, s->Mp16, s->t16, s->r32, st);
         if (e == cudaSuccess) e = finish_on(s, kBeta, st);
         if (e == cudaSuccess) {
             launch_pdl(cg_xpay_h<FMT>, dim3(nb), kThreads, st, static_cast<const float4 *>(s->r32),
-                       static_cast<char *>(s->p16), (const Scalars *)s->sc, g.Vh, g.stride);
+                       static_cast<float4 *>(s->e32), static_cast<char *>(s->p16), (const Scalars *)s->sc, g.Vh, g.stride);
             count_launch();
             e = cudaGetLastError();
         }
@@ -596,7 +561,7 @@ cudaError_t zero(gbds_solver s, void *v, cudaStream_t st) {
 void release(gbds_solver s) {
     void *bufs[] = {s->gauge64, s->gauge32, s->gauge_df, s->xdf, s->b64, s->c64, s->x64, s->r64, s->p64, s->Ap64,
                     s->Mp64, s->t64,
-                    s->e32, s->r32, s->p32, s->Ap32, s->Mp32, s->t32, s->p16, s->Ap16, s->Mp16, s->t16, s->gauge16,
+                    s->e32, s->r32, s->p32, s->Mp32, s->t32, s->p16, s->Mp16, s->t16, s->gauge16,
                     s->partials, s->sc};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -627,7 +592,7 @@ extern "C" int gbds_solver_create(gbds_solver *out, const int dims[4], const gbd
     for (void **b : d64)
         if (e == cudaSuccess) e = cudaMalloc(b, f64);
     if (p->inner_prec == 32) {
-        void **d32[] = {&s->e32, &s->r32, &s->p32, &s->Ap32, &s->Mp32, &s->t32};
+        void **d32[] = {&s->e32, &s->r32, &s->p32, &s->Mp32, &s->t32};
         for (void **b : d32)
             if (e == cudaSuccess) e = cudaMalloc(b, f32);
         if (e == cudaSuccess) e = cudaMalloc(&s->gauge32, gauge_bytes(g, 32, p->inner_recon));
@@ -637,7 +602,7 @@ extern "C" int gbds_solver_create(gbds_solver *out, const int dims[4], const gbd
         void **d32[] = {&s->e32, &s->r32, &s->Mp32, &s->t32};
         for (void **b : d32)
             if (e == cudaSuccess) e = cudaMalloc(b, f32);
-        void **d16[] = {&s->p16, &s->Ap16, &s->Mp16, &s->t16};
+        void **d16[] = {&s->p16, &s->Mp16, &s->t16};
         for (void **b : d16)
             if (e == cudaSuccess) e = cudaMalloc(b, f16);
         if (e == cudaSuccess) e = cudaMalloc(&s->gauge32, gauge_bytes(g, 32, p->inner_recon));
@@ -783,7 +748,7 @@ static int solve_mixed(gbds_solver s, const double *b_packed, double *x_packed, 
         if (need > delta) delta = need;
         int it = 0;
         if (!half)
-            e = cg<float>(s, s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Ap32, s->Mp32, s->t32,
+            e = cg<float>(s, s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Mp32, s->t32,
                           delta * delta, s->prm.max_iter - total, &it, st);
         else if (s->fmt16 == kFmtF16N)
             e = cg_h<kFmtF16N>(s, delta * delta, s->prm.max_iter - total, &it, st);
@@ -851,7 +816,7 @@ static int solve_impl(gbds_solver s, const double *b_packed, double *x_packed, g
             e = norm_into<double>(s, s->c64, s->r64, s->p64, kSetRR, st);
             int it = 0;
             if (e == cudaSuccess)
-                e = cg<double>(s, s->gauge64, 18, s->x64, s->r64, s->p64, s->Ap64, s->Mp64, s->t64, tol2 * c2,
+                e = cg<double>(s, s->gauge64, 18, s->x64, s->r64, s->p64, s->Mp64, s->t64, tol2 * c2,
                                s->prm.max_iter, &it, st);
             total = it;
             out.cycles = 1;
@@ -885,7 +850,7 @@ static int solve_impl(gbds_solver s, const double *b_packed, double *x_packed, g
                 if (need > delta) delta = need;
                 int it = 0;
                 if (!half)
-                    e = cg<float>(s, s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Ap32, s->Mp32, s->t32,
+                    e = cg<float>(s, s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Mp32, s->t32,
                                   delta * delta, s->prm.max_iter - total, &it, st);
                 else if (s->fmt16 == kFmtF16N)
                     e = cg_h<kFmtF16N>(s, delta * delta, s->prm.max_iter - total, &it, st);
