@@ -178,13 +178,14 @@ int gbds_op_dslash(gbds_op op, const void *gauge, const void *psi, void *res,
  * accepted and runs the one kernel.  Several rhs or 16-bit storage: 0 = the plain
  * multi-RHS kernel, 1 = the packed FP32x2 form (8, 16, 32 rhs; the block
  * size is fixed at 128), 2 = projection, multiply and reconstruction all in
- * packed FP32x2 (8, 16, 32 rhs; 128-thread blocks; every storage format),
- * 3 = variant 2 with two rhs per thread, which share each staged link (the
- * default from 16 rhs on for both FP32 layouts), and for the 16-bit formats
- * 4 = variant 3 with each thread's neighbour spinors prefetched two hops
- * ahead by cp.async into shared memory (their default from 16 rhs on).
- * Variants 1 to 4 run the plain kernel for other counts of rhs (variant 4 on
- * the FP32 formats runs variant 3).
+ * packed FP32x2 (2 rhs and more; 128-thread blocks; every storage format),
+ * 3 = variant 2 with two rhs per thread, which share each staged link (FP32: 8,
+ * 16, 32 rhs; 16-bit formats: any even count from 4, other than 8, 16, 32 with
+ * fields aligned to 32 bytes), and for the 16-bit formats 4 = variant 3 with
+ * each thread's neighbour spinors prefetched two hops ahead by cp.async into
+ * shared memory (8, 16, 32 rhs).  Where variant 4 does not apply, variant 3
+ * runs, else variant 2, else the plain kernel (1 rhs, or variant 1 with another
+ * count).  The default follows the count and the format.
  * gbds_op_num_variants gives the count.  Used by the autotuner. */
 int gbds_op_set_tuning(gbds_op op, int threads, int variant);
 int gbds_op_get_tuning(gbds_op op, int *threads, int *variant);

@@ -116,6 +116,30 @@ extern "C" int gbds_op_create(gbds_op *op, const int dims[4], int nd, int prec, 
     return gbds_op_create_ex(op, dims, nd, prec, recon, 1, GBDS_SPINOR_NATIVE);
 }
 
+// The multi-RHS kernel for a count and storage format.  What decides is how
+// many rhs share a staged link against what the staging and its barrier cost,
+// and for 16-bit storage the conversions, which the packed kernels write
+// straight into their pairs.  us at 24^3x48, 18-real links, plain kernel /
+// chosen one:
+//   FP32 (native)     4: 105 / 105   6: 149 / 149  12: 275 / 261
+//                    16: 360 / 284  24: 549 / 491  32: 721 / 568
+//   bfloat16          4:  91 /  91   6: 132 / 120  12: 250 / 198
+//                    16: 325 / 213  24: 485 / 358  32: 632 / 405
+//   half + norm       4: 123 /  96   6: 168 / 129  12: 316 / 223
+//                    16: 424 / 254  24: 603 / 415  32: 807 / 491
+// (odd counts: the two-rhs kernels do not apply; FP32 9: 216 / 217, bfloat16 7:
+// 151 with the plain kernel, 147 packed, half + norm 5: 144 / 121).  With 8 rhs
+// the default stays the plain kernel (half + norm: variant 2); gbds_op_autotune
+// or gbds_op_set_tuning reach the packed ones (FP32 193 / 166, bfloat16 172 / 133).
+static int gen_variant(int nrhs, int format) {
+    const bool bf16 = format == GBDS_SPINOR_BF16, half = bf16 || format == GBDS_SPINOR_F16_NORM;
+    if (nrhs == 16 || nrhs == 32) return half ? 4 : 3;
+    if (nrhs == 8) return format == GBDS_SPINOR_F16_NORM ? 2 : 0;
+    if (!half) return nrhs >= 8 ? 2 : 0;
+    if (nrhs % 2 == 0 && nrhs >= 6) return 3;
+    return nrhs >= (bf16 ? 9 : 4) ? 2 : 0;
+}
+
 extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int prec, int recon, int nrhs, int format) {
     if (!op) return set_error(GBDS_ERROR_INVALID_VALUE, "op is NULL");
     *op = nullptr;
@@ -151,13 +175,7 @@ extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int pre
     // rhs a thread, 4 = 3 with cp.async prefetching (16-bit storage);
     // autotune chooses per shape.
     const bool gen = nrhs > 1 || (format != GBDS_SPINOR_NATIVE && format != GBDS_SPINOR_DOUBLE_FLOAT);
-    // from 16 rhs on: for 16-bit storage the fully packed kernel with two rhs
-    // a thread and cp.async prefetching (variant 4), for both FP32 layouts
-    // the same without prefetching (3)
-    const int gen_variant =
-        nrhs >= 16 ? (format == GBDS_SPINOR_BF16 || format == GBDS_SPINOR_F16_NORM ? 4 : 3)
-                   : (nrhs == 8 && format == GBDS_SPINOR_F16_NORM ? 2 : 0);  // 24^3x48, 8 rhs: 0.226 -> 0.182 ms
-    o->variant = gen ? gen_variant : ((prec == 32 && recon == 18) ? 1 : 0);
+    o->variant = gen ? gen_variant(nrhs, format) : ((prec == 32 && recon == 18) ? 1 : 0);
     if (gen) o->g.zblock = gen_zblock(g, nrhs, format, recon);
     o->tensor_cores = 0;
     o->d_err = nullptr;

@@ -598,36 +598,14 @@ __device__ __forceinline__ void packed_hop(const float (&v)[24], float nrm, cons
     }
 }
 
-template <int FMT, int RECON, int ISIGN, int NRHS, int EPI>
-__global__ void __launch_bounds__(128, 5) dslash_gen3_kernel(const GenArgs a) {
-    static_assert(NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides");
-    pdl_allow_next();
-    pdl_wait_prev();
-    constexpr int P = 128 / NRHS;  // sites per CTA
-    constexpr bool SCALE = FMT == kFmtF16N;
-    __shared__ float2 sL[P][8][9];  // (Mr, Mi) splats
-    const int t = threadIdx.x;
-    const int p = t / NRHS, r = t % NRHS;
-    const int h = gen_site(a.g, blockIdx.x * P + p);
-    const bool act = h < a.g.Vh;
-    if constexpr (EPI >= 2 && FMT == kFmtF32Pairs) {
-        // the epilogue's operands (x, and r for the CG update) toward L2 now:
-        // their loads come after the hops, at the end of the thread
-        if (act) {
-            const size_t i = (size_t)h * NRHS + r;
-#pragma unroll
-            for (int k = 0; k < 6; k++) {
-                prefetch_l2(reinterpret_cast<const float4 *>(a.x) + (size_t)k * a.cs + i);
-                if constexpr (EPI == 3) prefetch_l2(a.rvec + (size_t)k * a.cs + i);
-            }
-        }
-    }
-    Nbr n;
-    if (act) neighbours<4>(a.g, h, a.pt, n);
-    if (act && r < 8) {
-        // link r of the site: direction r / 2, forward (even r) or backward
-        const int mu = r >> 1;
-        const bool bwd = r & 1;
+// Stage the links l = r, r + step, ... < 8 of site h as (Mr, Mi) of M = U
+// (forward, even l; direction l / 2) or U^dagger (backward).
+template <int RECON>
+__device__ __forceinline__ void stage_links(const GenArgs &a, const Nbr &n, int h, int r, int step, bool act,
+                                            float2 (*sL)[8][9]) {
+    for (int l = r; act && l < 8; l += step) {
+        const int mu = l >> 1;
+        const bool bwd = l & 1;
         const int nbm = mu == 0 ? n.b[0] : (mu == 1 ? n.b[1] : (mu == 2 ? n.b[2] : n.b[3]));
         const int lp = bwd ? 1 - a.pt : a.pt;
         cx<float> U[3][3];
@@ -640,9 +618,60 @@ __global__ void __launch_bounds__(128, 5) dslash_gen3_kernel(const GenArgs a) {
                 // forward: M_ij = U_ij; backward: M_ij = conj(U_ji)
                 const float mr = bwd ? U[j][i].r : U[i][j].r;
                 const float mi = bwd ? -U[j][i].i : U[i][j].i;
-                sL[p][r][i * 3 + j] = make_float2(mr, mi);
+                (*sL)[l][i * 3 + j] = make_float2(mr, mi);
             }
     }
+}
+
+// Shared memory of the staged links, (Mr, Mi) of 8 links a site: SITES sites,
+// or (0) as many as the launch gave.
+template <int SITES>
+__device__ __forceinline__ float2 (*staged_links())[8][9] {
+    if constexpr (SITES > 0) {
+        __shared__ float2 s[SITES][8][9];
+        return s;
+    } else {
+        extern __shared__ __align__(16) unsigned char dyn[];
+        return reinterpret_cast<float2 (*)[8][9]>(dyn);
+    }
+}
+
+// One rhs a thread.  NRHS 0: any count from 2 at run time (128 / nrhs sites a
+// CTA, the remaining threads idle).  Bound by the latency of the spinor loads
+// (long scoreboard 5.4 of 8.5 stall cycles an instruction at 20 warps per SM,
+// L1 data pipe 76 %, FMA pipe 42 %), so registers are capped for 28 warps:
+// 24^3x48, 16 rhs, FP32 0.320 -> 0.308 ms, FP32 pairs 0.308 -> 0.297 (prefetching
+// the next hop into registers at 12 or 16 warps: 0.340-0.391), BF16 8 rhs 0.150
+// -> 0.138; half + norm with a compile-time count keeps 20 warps (8 rhs 0.153
+// against 0.166).
+template <int FMT, int RECON, int ISIGN, int NRHS, int EPI>
+__global__ void __launch_bounds__(128, FMT == kFmtF16N && NRHS ? 5 : 7) dslash_gen3_kernel(const GenArgs a) {
+    static_assert(NRHS == 0 ? EPI == 0 : NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides, or any count");
+    pdl_allow_next();
+    pdl_wait_prev();
+    const int nr = nrhs_of<NRHS>(a);
+    const int P = 128 / nr;  // sites per CTA
+    constexpr bool SCALE = FMT == kFmtF16N;
+    float2 (*sL)[8][9] = staged_links<NRHS ? 128 / (NRHS ? NRHS : 1) : 0>();
+    const int t = threadIdx.x;
+    const int p = t / nr, r = t % nr;
+    const int h = gen_site(a.g, blockIdx.x * P + p);
+    const bool act = h < a.g.Vh && (NRHS || p < P);
+    if constexpr (EPI >= 2 && FMT == kFmtF32Pairs) {
+        // the epilogue's operands (x, and r for the CG update) toward L2 now:
+        // their loads come after the hops, at the end of the thread
+        if (act) {
+            const size_t i = (size_t)h * nr + r;
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                prefetch_l2(reinterpret_cast<const float4 *>(a.x) + (size_t)k * a.cs + i);
+                if constexpr (EPI == 3) prefetch_l2(a.rvec + (size_t)k * a.cs + i);
+            }
+        }
+    }
+    Nbr n;
+    if (act) neighbours<4>(a.g, h, a.pt, n);
+    stage_links<RECON>(a, n, h, r, nr, act, sL + p);
     __syncthreads();
     float nrm = 0.f;
     if (act) {
@@ -652,9 +681,9 @@ __global__ void __launch_bounds__(128, 5) dslash_gen3_kernel(const GenArgs a) {
 #define GBDS_G3_HOP(MU, LORD)                                                                            \
     {                                                                                                    \
         float v[24];                                                                                     \
-        float sc = load_reals<FMT>(a.psi, a.cs, (size_t)n.f[MU] * NRHS + r, v);                          \
+        float sc = load_reals<FMT>(a.psi, a.cs, (size_t)n.f[MU] * nr + r, v);                          \
         packed_hop<MU, ISIGN, LORD, SCALE>(v, sc, sL[p][2 * MU], UR, UI, LR, LI);                        \
-        sc = load_reals<FMT>(a.psi, a.cs, (size_t)n.b[MU] * NRHS + r, v);                                \
+        sc = load_reals<FMT>(a.psi, a.cs, (size_t)n.b[MU] * nr + r, v);                                \
         packed_hop<MU, -ISIGN, LORD, SCALE>(v, sc, sL[p][2 * MU + 1], UR, UI, LR, LI);                   \
     }
         GBDS_G3_HOP(0, 1)
@@ -675,7 +704,7 @@ __global__ void __launch_bounds__(128, 5) dslash_gen3_kernel(const GenArgs a) {
             acc[2][c] = {LR[c].x, LI[c].x};
             acc[3][c] = {LR[c].y, LI[c].y};
         }
-        const size_t i = (size_t)h * NRHS + r;
+        const size_t i = (size_t)h * nr + r;
         if constexpr (EPI == 3) {
             static_assert(FMT == kFmtF32Pairs, "the fused CG update works on FP32 spin pairs");
             const RhsCgScalars &sq = a.rsc[r];
@@ -820,26 +849,7 @@ __global__ void __launch_bounds__(128, 4) dslash_gen4_kernel(const GenArgs a) {
     const bool act = h < a.g.Vh;
     Nbr n;
     if (act) neighbours<4>(a.g, h, a.pt, n);
-    // links l = r, r + H, ... < 8 of the site (H = 4 threads a site for 8 rhs):
-    // direction l / 2, forward (even l) or backward
-    for (int l = r; act && l < 8; l += H) {
-        const int mu = l >> 1;
-        const bool bwd = l & 1;
-        const int nbm = mu == 0 ? n.b[0] : (mu == 1 ? n.b[1] : (mu == 2 ? n.b[2] : n.b[3]));
-        const int lp = bwd ? 1 - a.pt : a.pt;
-        cx<float> U[3][3];
-        Field<float>::template load_link<RECON>(a.gauge + (size_t)(lp * 4 + mu) * a.link_block_bytes, a.g.stride,
-                                                bwd ? nbm : h, U);
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                // forward: M_ij = U_ij; backward: M_ij = conj(U_ji)
-                const float mr = bwd ? U[j][i].r : U[i][j].r;
-                const float mi = bwd ? -U[j][i].i : U[i][j].i;
-                sL[p][l][i * 3 + j] = make_float2(mr, mi);
-            }
-    }
+    stage_links<RECON>(a, n, h, r, H, act, sL + p);  // H = 4 threads a site for 8 rhs
     __syncthreads();
     if (!act) return;
     float2 UR[2][3], UI[2][3], LR[2][3], LI[2][3];
@@ -884,6 +894,118 @@ __global__ void __launch_bounds__(128, 4) dslash_gen4_kernel(const GenArgs a) {
             acc[3][c] = {LR[q][c].y, LI[q][c].y};
         }
         Sio<FMT>::store(a.res, a.cs, (size_t)h * NRHS + r + q * H, acc);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Two adjacent rhs a thread, 16-bit storage, any even count from 4 at run time
+// (variant 3 for the counts other than 16 and 32): rhs 2 r and 2 r + 1 lie in 32
+// consecutive bytes of every component, one 256-bit load, and a warp's loads
+// are one contiguous run also where the threads of a site do not divide the
+// warp.  24^3x48, us, against one rhs a thread (variant 2) and the plain kernel:
+// BF16 12 rhs 198 / 219 / 250, half + norm 12 rhs 223 / 240 / 316, BF16 24 rhs
+// 358 / 391 / 485.
+// (For 16 and 32 rhs, and for FP32 storage, the eight-register operands of the
+// loads cost more than they save: BF16 16 rhs 226 against 213 with variant 4,
+// FP32 16 rhs 316 against 284 with the two-rhs kernel above.)
+// ---------------------------------------------------------------------------
+
+// 32 bytes at a 32-byte aligned address.
+__device__ __forceinline__ void ldg32(const void *p, unsigned (&v)[8]) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+}
+
+// The 24 reals of the rhs at elements i (even) and i + 1, as load_reals.
+template <int FMT>
+__device__ __forceinline__ void load_reals2(const char *base, size_t cs, size_t i, float (&v)[2][24], float (&sc)[2]) {
+    static_assert(FMT == kFmtBF16 || FMT == kFmtF16N, "16-bit storage");
+    const char *p = base + i * 16;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        unsigned w[8];
+        ldg32(p + (size_t)k * cs * 16, w);
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const unsigned u = w[4 * q + c];
+                if constexpr (FMT == kFmtBF16) {
+                    v[q][8 * k + 2 * c] = __uint_as_float(u << 16);
+                    v[q][8 * k + 2 * c + 1] = __uint_as_float(u & 0xffff0000u);
+                } else {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&u));
+                    v[q][8 * k + 2 * c] = f.x;
+                    v[q][8 * k + 2 * c + 1] = f.y;
+                }
+            }
+    }
+    sc[0] = sc[1] = 1.f;
+    if constexpr (FMT == kFmtF16N) {
+        const float2 n = __ldg(reinterpret_cast<const float2 *>(Sio<kFmtF16N>::norms(base, cs) + i));
+        sc[0] = n.x;
+        sc[1] = n.y;
+    }
+}
+
+template <int FMT, int RECON, int ISIGN>
+__global__ void __launch_bounds__(128, 4) dslash_gen4w_kernel(const GenArgs a) {
+    pdl_allow_next();
+    pdl_wait_prev();
+    const int nr = a.nrhs, H = nr / 2, P = 128 / H;  // threads per site, sites per CTA
+    constexpr bool SCALE = FMT == kFmtF16N;
+    float2 (*sL)[8][9] = staged_links<0>();
+    const int t = threadIdx.x;
+    const int p = t / H, r = t % H;
+    const int h = gen_site(a.g, blockIdx.x * P + p);
+    const bool act = h < a.g.Vh && p < P;
+    Nbr n;
+    if (act) neighbours<4>(a.g, h, a.pt, n);
+    stage_links<RECON>(a, n, h, r, H, act, sL + p);
+    __syncthreads();
+    if (!act) return;
+    float2 UR[2][3], UI[2][3], LR[2][3], LI[2][3];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) UR[q][c] = UI[q][c] = LR[q][c] = LI[q][c] = make_float2(0.f, 0.f);
+#define GBDS_G4W_HOP(MU, LORD, NB, SIG, L)                                    \
+    {                                                                        \
+        float2 R[2][3], I[2][3];                                             \
+        float v[2][24], sc[2];                                               \
+        load_reals2<FMT>(a.psi, a.cs, (size_t)(NB) * nr + 2 * r, v, sc);     \
+        packed_project<MU, SIG, SCALE>(v[0], sc[0], R[0], I[0]);             \
+        packed_project<MU, SIG, SCALE>(v[1], sc[1], R[1], I[1]);             \
+        packed_mul_recon2<MU, SIG, LORD, true>(sL[p][L], R, I, UR, UI, LR, LI); \
+    }
+#define GBDS_G4W_DIR(MU, LORD)                      \
+    GBDS_G4W_HOP(MU, LORD, n.f[MU], ISIGN, 2 * MU) \
+    GBDS_G4W_HOP(MU, LORD, n.b[MU], -ISIGN, 2 * MU + 1)
+    GBDS_G4W_DIR(0, 1)
+    GBDS_G4W_DIR(1, 1)
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            LR[q][c] = make_float2(LR[q][c].y, LR[q][c].x);
+            LI[q][c] = make_float2(LI[q][c].y, LI[q][c].x);
+        }
+    GBDS_G4W_DIR(2, 0)
+    GBDS_G4W_DIR(3, 0)
+#undef GBDS_G4W_DIR
+#undef GBDS_G4W_HOP
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        cx<float> acc[4][3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            acc[0][c] = {UR[q][c].x, UI[q][c].x};
+            acc[1][c] = {UR[q][c].y, UI[q][c].y};
+            acc[2][c] = {LR[q][c].x, LI[q][c].x};
+            acc[3][c] = {LR[q][c].y, LI[q][c].y};
+        }
+        Sio<FMT>::store(a.res, a.cs, (size_t)h * nr + 2 * r + q, acc);
     }
 }
 
@@ -991,23 +1113,7 @@ __global__ void __launch_bounds__(128, G5Smem<FMT, NRHS>::MINB) dslash_gen5_kern
         if (act) g5_issue<FMT, NRHS, 1, 1>(a, n, r, ring, rnorm);
         cp_async_commit();
     }
-    for (int l = r; act && l < 8; l += H) {
-        const int mu = l >> 1;
-        const bool bwd = l & 1;
-        const int nbm = mu == 0 ? n.b[0] : (mu == 1 ? n.b[1] : (mu == 2 ? n.b[2] : n.b[3]));
-        const int lp = bwd ? 1 - a.pt : a.pt;
-        cx<float> U[3][3];
-        Field<float>::template load_link<RECON>(a.gauge + (size_t)(lp * 4 + mu) * a.link_block_bytes, a.g.stride,
-                                                bwd ? nbm : h, U);
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-                const float mr = bwd ? U[j][i].r : U[i][j].r;
-                const float mi = bwd ? -U[j][i].i : U[i][j].i;
-                sL[p][l][i * 3 + j] = make_float2(mr, mi);
-            }
-    }
+    stage_links<RECON>(a, n, h, r, H, act, sL + p);
     __syncthreads();
     if (!act) {
         cp_async_wait<0>();

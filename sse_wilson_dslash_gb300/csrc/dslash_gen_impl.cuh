@@ -123,6 +123,22 @@ void launch_gen4_nrhs(const GenArgs &a, int nrhs, cudaStream_t st) {
     }
 }
 
+// The kernels for any count: the links of 128 / (threads a site) sites are
+// staged in dynamic shared memory (at most 64 sites, 36 KB).
+template <int FMT, int RECON, int ISIGN>
+void launch_gen3_any(const GenArgs &a, int nrhs, cudaStream_t st) {
+    const unsigned vh = (unsigned)a.g.Vh, sites = 128 / nrhs;
+    launch_pdl_smem(dslash_gen3_kernel<FMT, RECON, ISIGN, 0, 0>, dim3((vh + sites - 1) / sites), 128,
+                    sites * 72 * sizeof(float2), st, a);
+}
+
+template <int FMT, int RECON, int ISIGN>
+void launch_gen4w(const GenArgs &a, int nrhs, cudaStream_t st) {
+    const unsigned vh = (unsigned)a.g.Vh, sites = 128 / (nrhs / 2);
+    launch_pdl_smem(dslash_gen4w_kernel<FMT, RECON, ISIGN>, dim3((vh + sites - 1) / sites), 128,
+                    sites * 72 * sizeof(float2), st, a);
+}
+
 // Variant 4 (16-bit storage): dynamic shared memory above the 48 KB default,
 // allowed once per kernel instance and device before its first launch there.
 template <int FMT, int RECON, int ISIGN, int NRHS>
@@ -172,21 +188,29 @@ cudaError_t launch_gen_t(const Geom &g, int recon, int nrhs, const void *gauge, 
     if (epi && (nrhs > 32 || (nrhs & (nrhs - 1)) != 0)) return cudaErrorInvalidValue;
     const bool packed_nrhs = nrhs == 8 || nrhs == 16 || nrhs == 32;
     const bool v2 = variant == 1 && packed_nrhs;
-    // variant 2 (fully packed, every format: the native FP32 layout holds
-    // the reals in order and the pairs are formed in registers; its xpay
-    // epilogue serves the batched solver's FP32-pair fields); like variant 1,
-    // it falls back to the plain kernel otherwise
-    const bool v3 = (variant >= 2 && variant <= 4) && packed_nrhs && (FMT == kFmtF32Pairs || !epi);
-    // variant 3: the fully packed kernel with two rhs per thread (no
-    // epilogue; with one, variant 2 runs); variant 4: the same with cp.async
-    // prefetching (16-bit storage; variant 3 for the FP32 formats)
-    const bool v5 = variant == 4 && packed_nrhs && (FMT == kFmtBF16 || FMT == kFmtF16N) && !epi;
+    // variant 2 (fully packed, one rhs a thread, every format and any count
+    // from 2; its xpay epilogue serves the batched solver's FP32-pair fields, 8,
+    // 16 or 32 rhs); like variant 1, it falls back to the plain kernel otherwise
+    const bool v3 = variant >= 2 && variant <= 4 && (epi ? packed_nrhs && FMT == kFmtF32Pairs : nrhs >= 2);
+    // variant 3: two rhs a thread (no epilogue), for 16-bit storage any even
+    // count from 4 (other than 16 and 32 with 256-bit loads, for fields aligned
+    // to them), for FP32 8, 16 and 32; variant 4: for 16-bit storage and 8, 16, 32
+    // rhs the same with cp.async prefetching; where these do not apply, variant 2
+    constexpr bool half = FMT == kFmtBF16 || FMT == kFmtF16N;
+    const bool aligned32 = ((reinterpret_cast<uintptr_t>(psi) | reinterpret_cast<uintptr_t>(res)) & 31u) == 0;
+    const bool v5 = variant == 4 && packed_nrhs && half && !epi;
+    const bool v4w = (variant == 3 || variant == 4) && half && nrhs >= 4 && nrhs % 2 == 0 && nrhs != 16 && nrhs != 32 &&
+                     aligned32 && !epi;
     const bool v4 = (variant == 3 || variant == 4) && packed_nrhs && !epi;
 #define GBDS_GEN(R, S)                                                   \
     do {                                                                 \
-        if constexpr (FMT == kFmtBF16 || FMT == kFmtF16N) {              \
+        if constexpr (half) {                                            \
             if (v5) {                                                    \
                 launch_gen5_nrhs<FMT, R, S>(a, nrhs, st);                \
+                break;                                                   \
+            }                                                            \
+            if (v4w) {                                                   \
+                launch_gen4w<FMT, R, S>(a, nrhs, st);                    \
                 break;                                                   \
             }                                                            \
         }                                                                \
@@ -196,11 +220,13 @@ cudaError_t launch_gen_t(const Geom &g, int recon, int nrhs, const void *gauge, 
         }                                                                \
         if (v3) {                                                        \
             if constexpr (FMT == kFmtF32Pairs) {                         \
-                if (epi) launch_gen3_nrhs<FMT, R, S, 2>(a, nrhs, st);    \
-                else launch_gen3_nrhs<FMT, R, S, 0>(a, nrhs, st);        \
-            } else {                                                     \
-                launch_gen3_nrhs<FMT, R, S, 0>(a, nrhs, st);             \
+                if (epi) {                                               \
+                    launch_gen3_nrhs<FMT, R, S, 2>(a, nrhs, st);         \
+                    break;                                               \
+                }                                                        \
             }                                                            \
+            if (packed_nrhs) launch_gen3_nrhs<FMT, R, S, 0>(a, nrhs, st); \
+            else launch_gen3_any<FMT, R, S>(a, nrhs, st);                \
             break;                                                       \
         }                                                                \
         if (v2 && epi) launch_gen2_nrhs<FMT, R, S, 2>(a, nrhs, st);      \

@@ -1188,30 +1188,36 @@ cudaError_t bfinish_on(gbds_bsolver b, int mode, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// the multi-RHS kernel of the launches without an epilogue (FP32 spin pairs,
+// 24^3x48: 8 rhs 0.167 ms with variant 2 against 0.197 with 3 and 0.194 plain,
+// 16 rhs 0.278 with 3 against 0.297 with 2)
+int packed_variant(gbds_bsolver b) { return b->nrhs >= 16 ? 3 : b->nrhs == 8 ? 2 : 0; }
+
 // out = in - kappa^2 D_eo D_oe in for all rhs (partials: per-rhs |out|^2)
 cudaError_t apply_Mb(gbds_bsolver b, const void *in, void *out, int isign, double *partials, cudaStream_t st) {
     gbds_solver s = b->s1;
     const float k2 = (float)(s->prm.kappa * s->prm.kappa);
-    // inner fields in FP32 spin pairs: the fully packed FP32x2 kernel from 16
-    // rhs on (measured faster there), two rhs a thread where there is no
-    // epilogue
-    const int v = b->nrhs >= 16 ? 2 : 0;
+    // inner fields in FP32 spin pairs: the fully packed FP32x2 kernel from 8
+    // rhs on (measured faster there), from 16 on with two rhs a thread where
+    // there is no epilogue
+    const int v = b->nrhs >= 8 ? 2 : 0;
     cudaError_t e = launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, in, b->t, isign, 0, nullptr, 0.f,
-                                    nullptr, st, v ? 3 : 0);
+                                    nullptr, st, packed_variant(b));
     if (e != cudaSuccess) return e;
     return launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, b->t, out, isign, 1, in, -k2, partials, st, v);
 }
 
-// The fully packed operator (16, 32 rhs) fuses the CG's r -= alpha Ap into
+// The fully packed operator (8, 16, 32 rhs) fuses the CG's r -= alpha Ap into
 // M^+'s second launch: Ap is never stored.
-bool fused_update(gbds_bsolver b) { return b->nrhs == 16 || b->nrhs == 32; }
+bool fused_update(gbds_bsolver b) { return b->nrhs >= 8; }
 
 // r -= alpha_r M^+ in for all active rhs, per-rhs |r|^2 partials
 cudaError_t apply_Mb_dagger_update(gbds_bsolver b, const void *in, cudaStream_t st) {
     gbds_solver s = b->s1;
     const float k2 = (float)(s->prm.kappa * s->prm.kappa);
     cudaError_t e =
-        launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, in, b->t, -1, 0, nullptr, 0.f, nullptr, st, 3);
+        launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, in, b->t, -1, 0, nullptr, 0.f, nullptr, st,
+                        packed_variant(b));
     if (e != cudaSuccess) return e;
     return launch_gen_f32p_cg_update(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, b->t, -1, 1, in, -k2, b->bsc, b->r,
                                      b->bpartials, st);
