@@ -174,7 +174,7 @@ int gbds_op_dslash(gbds_op op, const void *gauge, const void *psi, void *res,
 /* Launch tuning of gbds_op_dslash: threads per block (0 = default 128; a
  * multiple of 32 up to 256) and a kernel variant.  Single rhs: 0 = registers
  * uncapped; 1.. = variants that cap registers for more resident warps, which
- * launch 128-thread blocks; FP64 (native): every variant and block size is
+ * launch 128-thread blocks, and in FP32 the last one four warps a site; FP64 (native): every variant and block size is
  * accepted and runs the one kernel.  Several rhs or 16-bit storage: 0 = the plain
  * multi-RHS kernel, 1 = the packed FP32x2 form (8, 16, 32 rhs; the block
  * size is fixed at 128), 2 = projection, multiply and reconstruction all in

@@ -162,20 +162,17 @@ extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int pre
     o->g = g;
     o->prec = prec;
     o->recon = recon;
-    // Defaults from a sweep on GB300 at 32^3x64 and 24^3x48 (gbds_op_autotune
-    // refines them per lattice): FP32 recon 18 runs best with registers capped
-    // for 6 blocks of 128 threads per SM, FP32 recon 12 with 64-thread blocks,
-    // FP64 has one launch shape.
-    o->block = (prec == 32 && recon == 12) ? 64 : 128;
     o->nrhs = nrhs;
     o->format = format;
-    // Single rhs: the register-cap variant (see above).  Several rhs or
-    // another format: variant 0 = the plain multi-RHS kernel, 1 = its packed
+    // Single rhs, FP32: by the lattice (gbds_op_autotune refines it; FP64 has
+    // one launch shape).  Several rhs or another format: variant 0 = the plain multi-RHS kernel, 1 = its packed
     // FP32x2 colour multiply, 2 = the whole hop packed, 3 = the same with two
     // rhs a thread, 4 = 3 with cp.async prefetching (16-bit storage);
     // autotune chooses per shape.
     const bool gen = nrhs > 1 || (format != GBDS_SPINOR_NATIVE && format != GBDS_SPINOR_DOUBLE_FLOAT);
-    o->variant = gen ? gen_variant(nrhs, format) : ((prec == 32 && recon == 18) ? 1 : 0);
+    o->block = 128;
+    o->variant = gen ? gen_variant(nrhs, format) : 0;
+    if (!gen && prec == 32) f32_tuning(g, recon, &o->block, &o->variant);
     if (gen) o->g.zblock = gen_zblock(g, nrhs, format, recon);
     o->tensor_cores = 0;
     o->d_err = nullptr;

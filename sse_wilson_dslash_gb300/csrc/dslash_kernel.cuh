@@ -470,6 +470,82 @@ __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks) d
     Field<T>::store_spinor(a.res, a.g.stride, h, acc);
 }
 
+// ---------------------------------------------------------------------------
+// FP32, four warps a site (small lattices): of 32 consecutive sites warp 0
+// takes the forward hops of directions 0, 1, warp 1 the backward ones, warps 2
+// and 3 the same of directions 2, 3; the four sums are added up through shared
+// memory, each warp storing its share of the components.  Up to about 29 K
+// sites a checkerboard every site's CTA is resident at once (6 of 32 sites per
+// SM), and the time is the latency of one thread's chain of hops, two instead of
+// eight.  us a launch in a chain (18-real links; against one thread a site,
+// uncapped registers, and capped for 24 warps): 4^4 1.6 / 2.1 / 3.2, 8^4 1.7 /
+// 2.3 / 3.4, 12^3x24 3.6 / 4.3 / 6.3, 16^4 (above the line) 6.4 / 4.8 / 8.5.  Two
+// warps a site (forward and backward hops) were never the best.
+// ---------------------------------------------------------------------------
+
+template <int ND, int RECON, int ISIGN, int MU, bool BWD>
+__device__ __forceinline__ void split_hop(const DslashArgs<float> &a, int h, const Nbr &n, cx<float> (&acc)[4][3]) {
+    using F = Field<float>;
+    cx<float> s[4][3], hs[2][3], w[2][3], U[3][3];
+    const int nb = BWD ? n.b[MU] : n.f[MU], p = BWD ? 1 - a.pt : a.pt;
+    F::load_spinor(a.psi, a.g.stride, nb, s);
+    F::template load_link<RECON, true>(a.gauge + (size_t)(p * ND + MU) * a.link_block_bytes, a.g.stride, BWD ? nb : h, U);
+    project<MU, BWD ? -ISIGN : ISIGN>(s, hs);
+    su3_mul<BWD>(U, hs, w);
+    reconstruct<MU, BWD ? -ISIGN : ISIGN>(acc, w);
+}
+
+constexpr int kSplitSites = 32;  // sites per CTA
+
+template <int ND, int RECON, int ISIGN>
+__global__ void __launch_bounds__(128, 6) dslash_split_kernel(const DslashArgs<float> a) {
+    __shared__ float4 sm[4][6][32];
+    pdl_allow_next();
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int h = blockIdx.x * kSplitSites + lane;
+    const bool act = h < a.g.Vh;
+    Nbr n;
+    if (act) neighbours<ND>(a.g, h, a.pt, n);
+    pdl_wait_prev();
+    if (act) {
+        cx<float> acc[4][3];
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) acc[s][c] = {0.f, 0.f};
+        if (part == 0) {
+            split_hop<ND, RECON, ISIGN, 0, false>(a, h, n, acc);
+            split_hop<ND, RECON, ISIGN, 1, false>(a, h, n, acc);
+        } else if (part == 1) {
+            split_hop<ND, RECON, ISIGN, 0, true>(a, h, n, acc);
+            split_hop<ND, RECON, ISIGN, 1, true>(a, h, n, acc);
+        } else if (part == 2) {
+            split_hop<ND, RECON, ISIGN, 2, false>(a, h, n, acc);
+            if constexpr (ND == 4) split_hop<ND, RECON, ISIGN, 3, false>(a, h, n, acc);
+        } else {
+            split_hop<ND, RECON, ISIGN, 2, true>(a, h, n, acc);
+            if constexpr (ND == 4) split_hop<ND, RECON, ISIGN, 3, true>(a, h, n, acc);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            const cx<float> u = acc[(2 * k) / 3][(2 * k) % 3], v = acc[(2 * k + 1) / 3][(2 * k + 1) % 3];
+            sm[part][k][lane] = make_float4(u.r, u.i, v.r, v.i);
+        }
+    }
+    __syncthreads();
+    if (!act) return;
+    // warp p adds up and stores components p, p + 4, ... of the spinor
+    for (int k = part; k < 6; k += 4) {
+        float4 v = sm[0][k][lane];
+#pragma unroll
+        for (int q = 1; q < 4; q++) {
+            const float4 w = sm[q][k][lane];
+            v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+        }
+        __stcs(a.res + (size_t)k * a.g.stride + h, v);
+    }
+}
+
 // Register-cap variants: index -> MINB (see Bounds).
 template <typename T> struct Variants;
 template <> struct Variants<float> { static constexpr int n = 5; static constexpr int minb[5] = {0, 6, 7, 8, 10}; };

@@ -35,7 +35,9 @@ void count_launch(int n = 1);
 // Launchers (defined in dslash_f32.cu / dslash_f64.cu / layout.cu).
 // All pointers are device pointers; `stream` is a cudaStream_t.
 // block: threads per block (0 = default); variant: register-cap variant
-// (0 = uncapped; see Variants<T> in dslash_kernel.cuh).
+// (0 = uncapped; see Variants<T> in dslash_kernel.cuh), after them four warps a
+// site.  f32_tuning: the ones for a lattice.
+void f32_tuning(const Geom &g, int recon, int *block, int *variant);
 cudaError_t launch_dslash_f32(const Geom &g, int recon, const void *gauge, const void *psi,
                               void *res, int isign, int cb, int block, int variant, cudaStream_t stream);
 // FP64: one kernel and launch shape (dslash_f64.cu)

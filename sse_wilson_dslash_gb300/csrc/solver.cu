@@ -353,9 +353,11 @@ namespace {
 template <typename T>
 cudaError_t dslash(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign, int cb,
                    cudaStream_t st) {
-    if constexpr (sizeof(T) == 4) return launch_dslash_f32(g, recon, gauge, psi, res, isign, cb, recon == 12 ? 64 : 128,
-                                                           recon == 18 ? 1 : 0, st);
-    else return launch_dslash_f64(g, recon, gauge, psi, res, isign, cb, st);
+    if constexpr (sizeof(T) == 4) {
+        int block, variant;
+        f32_tuning(g, recon, &block, &variant);
+        return launch_dslash_f32(g, recon, gauge, psi, res, isign, cb, block, variant, st);
+    } else return launch_dslash_f64(g, recon, gauge, psi, res, isign, cb, st);
 }
 
 template <typename T>
