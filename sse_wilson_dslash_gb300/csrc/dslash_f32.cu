@@ -4,13 +4,25 @@
 namespace gbds {
 namespace {
 
-template <int ND, int RECON>
-cudaError_t launch_split(const DslashArgs<float> &a, int isign, cudaStream_t st) {
+template <int ND, int RECON, int EPI = 0>
+cudaError_t launch_split(const DslashArgs<float> &a, int isign, cudaStream_t st, const float4 *x = nullptr, float coef = 0.f,
+                         const CgUpdate<float> &upd = {}, double *partials = nullptr) {
     const dim3 grid((a.g.Vh + kSplitSites - 1) / kSplitSites);
-    if (isign > 0) launch_pdl(dslash_split_kernel<ND, RECON, 1>, grid, 128, st, a);
-    else launch_pdl(dslash_split_kernel<ND, RECON, -1>, grid, 128, st, a);
+    if (isign > 0) launch_pdl(dslash_split_kernel<ND, RECON, 1, EPI>, grid, 128, st, a, x, coef, upd, partials);
+    else launch_pdl(dslash_split_kernel<ND, RECON, -1, EPI>, grid, 128, st, a, x, coef, upd, partials);
     count_launch();
     return cudaGetLastError();
+}
+
+DslashArgs<float> f32_args(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int cb) {
+    DslashArgs<float> a;
+    a.g = g;
+    a.psi = static_cast<const float4 *>(psi);
+    a.res = static_cast<float4 *>(res);
+    a.gauge = static_cast<const char *>(gauge);
+    a.link_block_bytes = (size_t)recon * 4 * g.stride;
+    a.pt = 1 - cb;
+    return a;
 }
 
 // Four warps a site: the variant after the register caps.
@@ -53,27 +65,50 @@ void f32_tuning(const Geom &g, int recon, int *block, int *variant) {
 cudaError_t launch_dslash_f32(const Geom &g, int recon, const void *gauge, const void *psi, void *res,
                               int isign, int cb, int block, int variant, cudaStream_t stream) {
     if (variant == kSplitVariant) {
-        DslashArgs<float> a;
-        a.g = g;
-        a.psi = static_cast<const float4 *>(psi);
-        a.res = static_cast<float4 *>(res);
-        a.gauge = static_cast<const char *>(gauge);
-        a.link_block_bytes = (size_t)recon * 4 * g.stride;
-        a.pt = 1 - cb;
+        const DslashArgs<float> a = f32_args(g, recon, gauge, psi, res, cb);
         if (g.nd == 4) return recon == 18 ? launch_split<4, 18>(a, isign, stream) : launch_split<4, 12>(a, isign, stream);
         return recon == 18 ? launch_split<3, 18>(a, isign, stream) : launch_split<3, 12>(a, isign, stream);
     }
     return launch_dslash_t<float>(g, recon, gauge, psi, res, isign, cb, block, variant, stream);
 }
 int dslash_variants(int prec) { return prec == 32 ? Variants<float>::n + 1 : 3; }
+// The launches with an epilogue follow f32_tuning's first two lines (small
+// lattices), else registers capped for 6 CTAs per SM.
+namespace {
+
+template <bool UPD>
+cudaError_t launch_epilogue(const Geom &g, int recon, const void *gauge, const void *psi, const void *x, float coef, void *res,
+                            double *partials, int isign, int cb, cudaStream_t st, const CgUpdate<float> &upd = {}) {
+    int block, variant;
+    f32_tuning(g, recon, &block, &variant);
+    constexpr int EPI = UPD ? 2 : 1;
+    if (variant == kSplitVariant) {
+        const DslashArgs<float> a = f32_args(g, recon, gauge, psi, res, cb);
+        const float4 *xv = static_cast<const float4 *>(x);
+        return recon == 18 ? launch_split<4, 18, EPI>(a, isign, st, xv, coef, upd, partials)
+                           : launch_split<4, 12, EPI>(a, isign, st, xv, coef, upd, partials);
+    }
+    if (variant == 0)
+        return launch_dslash_xpay_t<float, UPD, 0, 0>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st, upd);
+    return launch_dslash_xpay_t<float, UPD>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st, upd);
+}
+
+}  // namespace
+
+int f32_partials(const Geom &g, int recon) {
+    int block, variant;
+    f32_tuning(g, recon, &block, &variant);
+    return variant == kSplitVariant ? (g.Vh + kSplitSites - 1) / kSplitSites : xpay_blocks(g);
+}
+
 cudaError_t launch_dslash_xpay_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
                                    float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream) {
-    return launch_dslash_xpay_t<float>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, stream);
+    return launch_epilogue<false>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, stream);
 }
 cudaError_t launch_dslash_cg_update_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
                                         float coef, const double *alpha, void *r, double *partials, int isign, int cb,
                                         cudaStream_t stream) {
-    return launch_dslash_xpay_t<float, true>(g, recon, gauge, psi, x, coef, nullptr, partials, isign, cb, stream,
-                                             {static_cast<float4 *>(r), alpha});
+    return launch_epilogue<true>(g, recon, gauge, psi, x, coef, nullptr, partials, isign, cb, stream,
+                                 {static_cast<float4 *>(r), alpha});
 }
 }  // namespace gbds

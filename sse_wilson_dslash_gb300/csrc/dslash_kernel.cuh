@@ -470,82 +470,6 @@ __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks) d
     Field<T>::store_spinor(a.res, a.g.stride, h, acc);
 }
 
-// ---------------------------------------------------------------------------
-// FP32, four warps a site (small lattices): of 32 consecutive sites warp 0
-// takes the forward hops of directions 0, 1, warp 1 the backward ones, warps 2
-// and 3 the same of directions 2, 3; the four sums are added up through shared
-// memory, each warp storing its share of the components.  Up to about 29 K
-// sites a checkerboard every site's CTA is resident at once (6 of 32 sites per
-// SM), and the time is the latency of one thread's chain of hops, two instead of
-// eight.  us a launch in a chain (18-real links; against one thread a site,
-// uncapped registers, and capped for 24 warps): 4^4 1.6 / 2.1 / 3.2, 8^4 1.7 /
-// 2.3 / 3.4, 12^3x24 3.6 / 4.3 / 6.3, 16^4 (above the line) 6.4 / 4.8 / 8.5.  Two
-// warps a site (forward and backward hops) were never the best.
-// ---------------------------------------------------------------------------
-
-template <int ND, int RECON, int ISIGN, int MU, bool BWD>
-__device__ __forceinline__ void split_hop(const DslashArgs<float> &a, int h, const Nbr &n, cx<float> (&acc)[4][3]) {
-    using F = Field<float>;
-    cx<float> s[4][3], hs[2][3], w[2][3], U[3][3];
-    const int nb = BWD ? n.b[MU] : n.f[MU], p = BWD ? 1 - a.pt : a.pt;
-    F::load_spinor(a.psi, a.g.stride, nb, s);
-    F::template load_link<RECON, true>(a.gauge + (size_t)(p * ND + MU) * a.link_block_bytes, a.g.stride, BWD ? nb : h, U);
-    project<MU, BWD ? -ISIGN : ISIGN>(s, hs);
-    su3_mul<BWD>(U, hs, w);
-    reconstruct<MU, BWD ? -ISIGN : ISIGN>(acc, w);
-}
-
-constexpr int kSplitSites = 32;  // sites per CTA
-
-template <int ND, int RECON, int ISIGN>
-__global__ void __launch_bounds__(128, 6) dslash_split_kernel(const DslashArgs<float> a) {
-    __shared__ float4 sm[4][6][32];
-    pdl_allow_next();
-    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
-    const int h = blockIdx.x * kSplitSites + lane;
-    const bool act = h < a.g.Vh;
-    Nbr n;
-    if (act) neighbours<ND>(a.g, h, a.pt, n);
-    pdl_wait_prev();
-    if (act) {
-        cx<float> acc[4][3];
-#pragma unroll
-        for (int s = 0; s < 4; s++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) acc[s][c] = {0.f, 0.f};
-        if (part == 0) {
-            split_hop<ND, RECON, ISIGN, 0, false>(a, h, n, acc);
-            split_hop<ND, RECON, ISIGN, 1, false>(a, h, n, acc);
-        } else if (part == 1) {
-            split_hop<ND, RECON, ISIGN, 0, true>(a, h, n, acc);
-            split_hop<ND, RECON, ISIGN, 1, true>(a, h, n, acc);
-        } else if (part == 2) {
-            split_hop<ND, RECON, ISIGN, 2, false>(a, h, n, acc);
-            if constexpr (ND == 4) split_hop<ND, RECON, ISIGN, 3, false>(a, h, n, acc);
-        } else {
-            split_hop<ND, RECON, ISIGN, 2, true>(a, h, n, acc);
-            if constexpr (ND == 4) split_hop<ND, RECON, ISIGN, 3, true>(a, h, n, acc);
-        }
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            const cx<float> u = acc[(2 * k) / 3][(2 * k) % 3], v = acc[(2 * k + 1) / 3][(2 * k + 1) % 3];
-            sm[part][k][lane] = make_float4(u.r, u.i, v.r, v.i);
-        }
-    }
-    __syncthreads();
-    if (!act) return;
-    // warp p adds up and stores components p, p + 4, ... of the spinor
-    for (int k = part; k < 6; k += 4) {
-        float4 v = sm[0][k][lane];
-#pragma unroll
-        for (int q = 1; q < 4; q++) {
-            const float4 w = sm[q][k][lane];
-            v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
-        }
-        __stcs(a.res + (size_t)k * a.g.stride + h, v);
-    }
-}
-
 // Register-cap variants: index -> MINB (see Bounds).
 template <typename T> struct Variants;
 template <> struct Variants<float> { static constexpr int n = 5; static constexpr int minb[5] = {0, 6, 7, 8, 10}; };
@@ -709,6 +633,100 @@ __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks)
     }
 }
 
+// ---------------------------------------------------------------------------
+// FP32, four warps a site (small lattices): of 32 consecutive sites warp 0
+// takes the forward hops of directions 0, 1, warp 1 the backward ones, warps 2
+// and 3 the same of directions 2, 3; the four sums are added up through shared
+// memory, each warp storing its share of the components.  Up to about 29 K
+// sites a checkerboard every site's CTA is resident at once (6 of 32 sites per
+// SM), and the time is the latency of one thread's chain of hops, two instead of
+// eight.  us a launch in a chain (18-real links; against one thread a site,
+// uncapped registers, and capped for 24 warps): 4^4 1.6 / 2.1 / 3.2, 8^4 1.7 /
+// 2.3 / 3.4, 12^3x24 3.6 / 4.3 / 6.3, 16^4 (above the line) 6.4 / 4.8 / 8.5.  Two
+// warps a site (forward and backward hops) were never the best.  EPI 1, 2: the
+// epilogues of dslash_xpay_kernel (partials: one per CTA).
+// ---------------------------------------------------------------------------
+
+template <int ND, int RECON, int ISIGN, int MU, bool BWD>
+__device__ __forceinline__ void split_hop(const DslashArgs<float> &a, int h, const Nbr &n, cx<float> (&acc)[4][3]) {
+    using F = Field<float>;
+    cx<float> s[4][3], hs[2][3], w[2][3], U[3][3];
+    const int nb = BWD ? n.b[MU] : n.f[MU], p = BWD ? 1 - a.pt : a.pt;
+    F::load_spinor(a.psi, a.g.stride, nb, s);
+    F::template load_link<RECON, true>(a.gauge + (size_t)(p * ND + MU) * a.link_block_bytes, a.g.stride, BWD ? nb : h, U);
+    project<MU, BWD ? -ISIGN : ISIGN>(s, hs);
+    su3_mul<BWD>(U, hs, w);
+    reconstruct<MU, BWD ? -ISIGN : ISIGN>(acc, w);
+}
+
+constexpr int kSplitSites = 32;  // sites per CTA
+
+template <int ND, int RECON, int ISIGN, int EPI>
+__global__ void __launch_bounds__(128, 6)
+    dslash_split_kernel(const DslashArgs<float> a, const float4 *__restrict__ x, float coef, const CgUpdate<float> upd,
+                        double *partials) {
+    __shared__ float4 sm[4][6][32];
+    pdl_allow_next();
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int h = blockIdx.x * kSplitSites + lane;
+    const bool act = h < a.g.Vh;
+    Nbr n;
+    if (act) neighbours<ND>(a.g, h, a.pt, n);
+    pdl_wait_prev();
+    if (act) {
+        cx<float> acc[4][3];
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) acc[s][c] = {0.f, 0.f};
+        if (part == 0) {
+            split_hop<ND, RECON, ISIGN, 0, false>(a, h, n, acc);
+            split_hop<ND, RECON, ISIGN, 1, false>(a, h, n, acc);
+        } else if (part == 1) {
+            split_hop<ND, RECON, ISIGN, 0, true>(a, h, n, acc);
+            split_hop<ND, RECON, ISIGN, 1, true>(a, h, n, acc);
+        } else if (part == 2) {
+            split_hop<ND, RECON, ISIGN, 2, false>(a, h, n, acc);
+            if constexpr (ND == 4) split_hop<ND, RECON, ISIGN, 3, false>(a, h, n, acc);
+        } else {
+            split_hop<ND, RECON, ISIGN, 2, true>(a, h, n, acc);
+            if constexpr (ND == 4) split_hop<ND, RECON, ISIGN, 3, true>(a, h, n, acc);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            const cx<float> u = acc[(2 * k) / 3][(2 * k) % 3], v = acc[(2 * k + 1) / 3][(2 * k + 1) % 3];
+            sm[part][k][lane] = make_float4(u.r, u.i, v.r, v.i);
+        }
+    }
+    __syncthreads();
+    float nrm = 0.f;
+    // warp p adds up and stores components p, p + 4, ... of the spinor
+    for (int k = part; act && k < 6; k += 4) {
+        float4 v = sm[0][k][lane];
+#pragma unroll
+        for (int q = 1; q < 4; q++) {
+            const float4 w = sm[q][k][lane];
+            v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+        }
+        const size_t i = (size_t)k * a.g.stride + h;
+        if constexpr (EPI) {
+            const float4 xv = __ldg(x + i);
+            v = make_float4(fmaf(coef, v.x, xv.x), fmaf(coef, v.y, xv.y), fmaf(coef, v.z, xv.z), fmaf(coef, v.w, xv.w));
+            if constexpr (EPI == 2) {
+                const float al = -(float)*upd.alpha;
+                const float4 r = upd.r[i];
+                v = make_float4(fmaf(al, v.x, r.x), fmaf(al, v.y, r.y), fmaf(al, v.z, r.z), fmaf(al, v.w, r.w));
+            }
+            nrm += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        }
+        if constexpr (EPI == 2) upd.r[i] = v;
+        else __stcs(a.res + i, v);
+    }
+    if constexpr (EPI) {
+        if (partials) block_sum_to<float>(partials, nrm);
+    }
+}
+
 template <typename T> struct XpayMinb;
 template <> struct XpayMinb<float> { static constexpr int r18 = 6, r12 = 6; };
 template <> struct XpayMinb<dfloat> { static constexpr int r18 = 4, r12 = 4; };
@@ -716,7 +734,7 @@ template <> struct XpayMinb<dfloat> { static constexpr int r18 = 4, r12 = 4; };
 // Grid blocks of an xpay launch (the size `partials` must have).
 inline int xpay_blocks(const Geom &g) { return (g.Vh + 127) / 128; }
 
-template <typename T, bool UPD = false>
+template <typename T, bool UPD = false, int M18 = XpayMinb<T>::r18, int M12 = XpayMinb<T>::r12>
 cudaError_t launch_dslash_xpay_t(const Geom &g, int recon, const void *gauge, const void *psi, const void *x, T coef,
                                  void *res, double *partials, int isign, int cb, cudaStream_t stream,
                                  const CgUpdate<T> &upd = {}) {
@@ -730,13 +748,12 @@ cudaError_t launch_dslash_xpay_t(const Geom &g, int recon, const void *gauge, co
     a.pt = 1 - cb;
     const dim3 grid(xpay_blocks(g));
     const auto *xv = static_cast<const typename VecOf<T>::S *>(x);
-    constexpr int m18 = XpayMinb<T>::r18, m12 = XpayMinb<T>::r12;
     if (recon == 18) {
-        if (isign > 0) launch_pdl(dslash_xpay_kernel<T, 18, 1, m18, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
-        else launch_pdl(dslash_xpay_kernel<T, 18, -1, m18, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
+        if (isign > 0) launch_pdl(dslash_xpay_kernel<T, 18, 1, M18, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
+        else launch_pdl(dslash_xpay_kernel<T, 18, -1, M18, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
     } else {
-        if (isign > 0) launch_pdl(dslash_xpay_kernel<T, 12, 1, m12, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
-        else launch_pdl(dslash_xpay_kernel<T, 12, -1, m12, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
+        if (isign > 0) launch_pdl(dslash_xpay_kernel<T, 12, 1, M12, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
+        else launch_pdl(dslash_xpay_kernel<T, 12, -1, M12, UPD>, grid, 128, stream, a, xv, coef, upd, partials);
     }
     count_launch();
     return cudaGetLastError();

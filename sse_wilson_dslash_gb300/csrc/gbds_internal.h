@@ -47,8 +47,9 @@ cudaError_t launch_dslash_f64(const Geom &g, int recon, const void *gauge, const
 int dslash_variants(int prec);
 
 // res = x + coef * Dslash(psi) (4D; res and x on checkerboard 1-cb); if
-// partials != nullptr, partials[b] = sum of |res|^2 over launch block b
-// (there are (Vh + 127) / 128 blocks).
+// partials != nullptr, partials[b] = sum of |res|^2 over launch block b (there
+// are (Vh + 127) / 128 blocks; FP32: f32_partials).
+int f32_partials(const Geom &g, int recon);
 cudaError_t launch_dslash_xpay_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
                                    float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream);
 // r -= alpha (x + coef * Dslash(psi)), alpha read on the device, with |r|^2 in

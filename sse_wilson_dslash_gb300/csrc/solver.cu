@@ -343,6 +343,7 @@ struct gbds_solver_s {
     double *partials = nullptr;
     Scalars *sc = nullptr;    // device
     Scalars *hsc = nullptr;   // pinned host copy
+    cudaEvent_t read = nullptr;  // the copy of a convergence test has arrived
     bool have_gauge = false;
 };
 
@@ -367,8 +368,9 @@ cudaError_t dslash_xpay(const Geom &g, int recon, const void *gauge, const void 
     else return launch_dslash_xpay_f64(g, gauge, psi, x, coef, res, partials, isign, cb, st);
 }
 
-cudaError_t finish_on(gbds_solver s, int mode, cudaStream_t st) {
-    launch_pdl(finish, dim3(1), 1024, st, s->partials, blocks(s->g), s->sc, mode);
+// n: the partials to add up (0: one per 128-site block)
+cudaError_t finish_on(gbds_solver s, int mode, cudaStream_t st, int n = 0) {
+    launch_pdl(finish, dim3(1), 1024, st, (const double *)s->partials, n ? n : blocks(s->g), s->sc, mode);
     count_launch();
     return cudaGetLastError();
 }
@@ -458,40 +460,67 @@ cudaError_t read_scalars(gbds_solver s, cudaStream_t st) {
     return e;
 }
 
-// CG on A = M^+ M with x, r, p prepared (x = 0, r = p = rhs, sc->rr = |rhs|^2).
-// Stops when rr <= target_rr or after max_iter iterations.
-template <typename T>
-cudaError_t cg(gbds_solver s, const void *gauge, int recon, void *x, void *r, void *p, void *Mp, void *t,
-               double target_rr, int max_iter, int *iters, cudaStream_t st) {
-    const Geom &g = s->g;
-    const int nb = blocks(g);
-    const int check_every = sizeof(T) == 4 ? 4 : 1;
+// The convergence test reads rr back every few iterations.  So that the GPU does
+// not idle while the host waits for it, the next iteration's first part (M p and
+// alpha, which write neither x nor r nor p) is enqueued behind the copy: unused
+// if the solve has converged.  On large lattices the unused part would cost more
+// than the wait (24^3x48: 100 us against 15), so there it follows the test.
+bool look_ahead(const Geom &g) { return blocks(g) <= 912; }
+
+// CG on A = M^+ M with x = 0, r = p = rhs, sc->rr = |rhs|^2 prepared.  first():
+// M p and alpha; second(): r -= alpha A p, beta, x += alpha p, p = r + beta p.
+// Stops when rr <= target_rr, after max_iter iterations, or (inner solves) when
+// it stagnates.
+template <typename FIRST, typename SECOND>
+cudaError_t cg_loop(gbds_solver s, const FIRST &first, const SECOND &second, int check_every, bool inner, double target_rr,
+                    int max_iter, int *iters, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     int k = 0;
     double best = 1e300;
     int best_k = 0;
+    bool ahead = false;  // first() of iteration k is already enqueued
     while (k < max_iter) {
-        e = apply_M<T>(s, gauge, recon, p, t, Mp, +1, s->partials, st);
-        if (e == cudaSuccess) e = finish_on(s, kAlpha, st);
-        if (e == cudaSuccess) e = apply_Mdag_update<T>(s, gauge, recon, Mp, t, r, st);
-        if (e == cudaSuccess) e = finish_on(s, kBeta, st);
-        if (e == cudaSuccess) {
-            launch_pdl(cg_xpay<T>, dim3(nb), kThreads, st, static_cast<const SV<T> *>(r), static_cast<SV<T> *>(x),
-                       static_cast<SV<T> *>(p), (const Scalars *)s->sc, g.Vh, g.stride);
-            count_launch();
-            e = cudaGetLastError();
-        }
+        if (!ahead) e = first();
+        ahead = false;
+        if (e == cudaSuccess) e = second();
         if (e != cudaSuccess) break;
         k++;
         if (k % check_every == 0 || k == max_iter) {
-            e = read_scalars(s, st);
+            e = cudaMemcpyAsync(s->hsc, s->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaEventRecord(s->read, st);
+            if (e == cudaSuccess && k < max_iter && look_ahead(s->g)) {
+                e = first();
+                ahead = true;
+            }
+            if (e == cudaSuccess) e = cudaEventSynchronize(s->read);
             if (e != cudaSuccess) break;
             if (!(s->hsc->rr > target_rr)) break;  // converged (or NaN: stop)
-            if (sizeof(T) == 4 && stagnated(s->hsc->rr, k, best, best_k)) break;
+            if (inner && stagnated(s->hsc->rr, k, best, best_k)) break;
         }
     }
     *iters = k;
     return e;
+}
+
+template <typename T>
+cudaError_t cg(gbds_solver s, const void *gauge, int recon, void *x, void *r, void *p, void *Mp, void *t, double target_rr,
+               int max_iter, int *iters, cudaStream_t st) {
+    const Geom &g = s->g;
+    const int parts = sizeof(T) == 4 ? f32_partials(g, recon) : 0;
+    auto first = [&] {
+        cudaError_t e = apply_M<T>(s, gauge, recon, p, t, Mp, +1, s->partials, st);
+        return e == cudaSuccess ? finish_on(s, kAlpha, st, parts) : e;
+    };
+    auto second = [&] {
+        cudaError_t e = apply_Mdag_update<T>(s, gauge, recon, Mp, t, r, st);
+        if (e == cudaSuccess) e = finish_on(s, kBeta, st, parts);
+        if (e != cudaSuccess) return e;
+        launch_pdl(cg_xpay<T>, dim3(blocks(g)), kThreads, st, static_cast<const SV<T> *>(r), static_cast<SV<T> *>(x),
+                   static_cast<SV<T> *>(p), (const Scalars *)s->sc, g.Vh, g.stride);
+        count_launch();
+        return cudaGetLastError();
+    };
+    return cg_loop(s, first, second, sizeof(T) == 4 ? 4 : 1, sizeof(T) == 4, target_rr, max_iter, iters, st);
 }
 
 // The 16-bit operator: out = in - kappa^2 D_eo D_oe in, FP16 links.
@@ -515,33 +544,20 @@ cudaError_t apply_Mdag_update_h(gbds_solver s, const void *in, void *tmp, void *
 template <int FMT>
 cudaError_t cg_h(gbds_solver s, double target_rr, int max_iter, int *iters, cudaStream_t st) {
     const Geom &g = s->g;
-    const int nb = blocks(g);
-    cudaError_t e = cudaSuccess;
-    int k = 0;
-    double best = 1e300;
-    int best_k = 0;
-    while (k < max_iter) {
-        e = apply_M_h(s, s->p16, s->t16, s->Mp16, +1, s->partials, st);
-        if (e == cudaSuccess) e = finish_on(s, kAlpha, st);
-        if (e == cudaSuccess) e = apply_Mdag_update_h(s, s->Mp16, s->t16, s->r32, st);
+    auto first = [&] {
+        cudaError_t e = apply_M_h(s, s->p16, s->t16, s->Mp16, +1, s->partials, st);
+        return e == cudaSuccess ? finish_on(s, kAlpha, st) : e;
+    };
+    auto second = [&] {
+        cudaError_t e = apply_Mdag_update_h(s, s->Mp16, s->t16, s->r32, st);
         if (e == cudaSuccess) e = finish_on(s, kBeta, st);
-        if (e == cudaSuccess) {
-            launch_pdl(cg_xpay_h<FMT>, dim3(nb), kThreads, st, static_cast<const float4 *>(s->r32),
-                       static_cast<float4 *>(s->e32), static_cast<char *>(s->p16), (const Scalars *)s->sc, g.Vh, g.stride);
-            count_launch();
-            e = cudaGetLastError();
-        }
-        if (e != cudaSuccess) break;
-        k++;
-        if (k % 4 == 0 || k == max_iter) {
-            e = read_scalars(s, st);
-            if (e != cudaSuccess) break;
-            if (!(s->hsc->rr > target_rr)) break;
-            if (stagnated(s->hsc->rr, k, best, best_k)) break;
-        }
-    }
-    *iters = k;
-    return e;
+        if (e != cudaSuccess) return e;
+        launch_pdl(cg_xpay_h<FMT>, dim3(blocks(g)), kThreads, st, static_cast<const float4 *>(s->r32),
+                   static_cast<float4 *>(s->e32), static_cast<char *>(s->p16), (const Scalars *)s->sc, g.Vh, g.stride);
+        count_launch();
+        return cudaGetLastError();
+    };
+    return cg_loop(s, first, second, 4, true, target_rr, max_iter, iters, st);
 }
 
 template <typename T>
@@ -568,6 +584,7 @@ void release(gbds_solver s) {
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (s->hsc) cudaFreeHost(s->hsc);
+    if (s->read) cudaEventDestroy(s->read);
 }
 
 }  // namespace
@@ -614,9 +631,11 @@ extern "C" int gbds_solver_create(gbds_solver *out, const int dims[4], const gbd
     const bool df = p->inner_prec != 64 && p->outer_double_float;
     if (e == cudaSuccess && df) e = cudaMalloc(&s->gauge_df, gauge_bytes(g, 64, 18));
     if (e == cudaSuccess && df) e = cudaMalloc(&s->xdf, f64);
-    if (e == cudaSuccess) e = cudaMalloc(&s->partials, sizeof(double) * (size_t)blocks(g));
+    const int parts = std::max(blocks(g), f32_partials(g, p->inner_recon));
+    if (e == cudaSuccess) e = cudaMalloc(&s->partials, sizeof(double) * (size_t)parts);
     if (e == cudaSuccess) e = cudaMalloc(&s->sc, sizeof(Scalars));
     if (e == cudaSuccess) e = cudaMallocHost(&s->hsc, sizeof(Scalars));
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->read, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         release(s);
         delete s;
@@ -720,7 +739,7 @@ static int solve_mixed(gbds_solver s, const double *b_packed, double *x_packed, 
         e = cudaGetLastError();
         if (e == cudaSuccess)
             e = apply_M<float>(s, s->gauge32, s->prm.inner_recon, s->r32, s->t32, s->Mp32, -1, s->partials, st);
-        if (e == cudaSuccess) e = finish_on(s, kNorm, st);
+        if (e == cudaSuccess) e = finish_on(s, kNorm, st, f32_partials(g, s->prm.inner_recon));
         if (e == cudaSuccess) e = read_scalars(s, st);
         if (e != cudaSuccess) break;
         const double s2 = s->hsc->norm;
