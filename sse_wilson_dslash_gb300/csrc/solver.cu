@@ -323,6 +323,17 @@ __global__ void f64_to_f32(const double *__restrict__ a, float *b, size_t n) {
 
 using namespace gbds;
 
+// kCheck iterations of an inner CG less their first part, recorded once per
+// solver (every buffer is the solver's own) and launched as one CUDA graph: a
+// small lattice's iteration is bound by the host's seven launches of about 3 us
+// each.  us an iteration, launched one by one / as a graph: 8^3x16 35.3 / 32.8, 16^3x32
+// 64.8 / 62.5, 24^3x48 202.6 / 201.2; 16 rhs on 16^3x32 38.0 / 37.5 ms a solve.
+constexpr int kCheck = 4;  // iterations between convergence tests
+struct IterGraph {
+    cudaGraphExec_t exec = nullptr;
+    int launches = 0;
+};
+
 struct gbds_solver_s {
     Geom g;
     gbds_solver_params prm;
@@ -344,6 +355,7 @@ struct gbds_solver_s {
     Scalars *sc = nullptr;    // device
     Scalars *hsc = nullptr;   // pinned host copy
     cudaEvent_t read = nullptr;  // the copy of a convergence test has arrived
+    IterGraph steps;             // the inner CG's
     bool have_gauge = false;
 };
 
@@ -460,6 +472,35 @@ cudaError_t read_scalars(gbds_solver s, cudaStream_t st) {
     return e;
 }
 
+// Record body(stream), which makes `launches` counted launches.  Where it cannot
+// be recorded, the graph stays empty and the iterations are launched one by one.
+template <typename BODY>
+void record(IterGraph &g, int launches, const BODY &body) {
+    cudaStream_t cs = nullptr;
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        const cudaError_t le = body(cs);
+        e = cudaStreamEndCapture(cs, &graph);
+        if (le != cudaSuccess) e = le;
+        else count_launch(-launches);  // recorded, not launched
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
+    if (e != cudaSuccess) {
+        g.exec = nullptr;
+        (void)cudaGetLastError();
+    }
+    if (graph) cudaGraphDestroy(graph);
+    if (cs) cudaStreamDestroy(cs);
+    g.launches = launches;
+}
+
+cudaError_t launch(const IterGraph &g, cudaStream_t st) {
+    count_launch(g.launches);
+    return cudaGraphLaunch(g.exec, st);
+}
+
 // The convergence test reads rr back every few iterations.  So that the GPU does
 // not idle while the host waits for it, the next iteration's first part (M p and
 // alpha, which write neither x nor r nor p) is enqueued behind the copy: unused
@@ -468,28 +509,35 @@ cudaError_t read_scalars(gbds_solver s, cudaStream_t st) {
 bool look_ahead(const Geom &g) { return blocks(g) <= 912; }
 
 // CG on A = M^+ M with x = 0, r = p = rhs, sc->rr = |rhs|^2 prepared.  first():
-// M p and alpha; second(): r -= alpha A p, beta, x += alpha p, p = r + beta p.
-// Stops when rr <= target_rr, after max_iter iterations, or (inner solves) when
-// it stagnates.
+// M p and alpha; second(): r -= alpha A p, beta, x += alpha p, p = r + beta p;
+// steps (where recorded): second() and kCheck - 1 whole iterations.  Stops when
+// rr <= target_rr, after max_iter iterations, or (inner solves) when it stagnates.
 template <typename FIRST, typename SECOND>
-cudaError_t cg_loop(gbds_solver s, const FIRST &first, const SECOND &second, int check_every, bool inner, double target_rr,
-                    int max_iter, int *iters, cudaStream_t st) {
+cudaError_t cg_loop(gbds_solver s, const FIRST &first, const SECOND &second, const IterGraph *steps, bool inner,
+                    double target_rr, int max_iter, int *iters, cudaStream_t st) {
+    const int check_every = inner ? kCheck : 1;
     cudaError_t e = cudaSuccess;
     int k = 0;
     double best = 1e300;
     int best_k = 0;
     bool ahead = false;  // first() of iteration k is already enqueued
     while (k < max_iter) {
-        if (!ahead) e = first();
+        if (!ahead) e = first(st);
         ahead = false;
-        if (e == cudaSuccess) e = second();
         if (e != cudaSuccess) break;
-        k++;
+        if (steps && steps->exec && k % kCheck == 0 && k + kCheck <= max_iter) {
+            e = launch(*steps, st);
+            k += kCheck;
+        } else {
+            e = second(st);
+            k++;
+        }
+        if (e != cudaSuccess) break;
         if (k % check_every == 0 || k == max_iter) {
             e = cudaMemcpyAsync(s->hsc, s->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaEventRecord(s->read, st);
             if (e == cudaSuccess && k < max_iter && look_ahead(s->g)) {
-                e = first();
+                e = first(st);
                 ahead = true;
             }
             if (e == cudaSuccess) e = cudaEventSynchronize(s->read);
@@ -502,25 +550,56 @@ cudaError_t cg_loop(gbds_solver s, const FIRST &first, const SECOND &second, int
     return e;
 }
 
+// The fields of one CG.
+struct CgFields {
+    const void *gauge;
+    int recon;
+    void *x, *r, *p, *Mp, *t;
+};
+
+CgFields inner_fields(gbds_solver s) {
+    return {s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Mp32, s->t32};
+}
+
+constexpr int kFirstLaunches = 3, kSecondLaunches = 4;  // of cg_first and cg_second
+
 template <typename T>
-cudaError_t cg(gbds_solver s, const void *gauge, int recon, void *x, void *r, void *p, void *Mp, void *t, double target_rr,
-               int max_iter, int *iters, cudaStream_t st) {
+cudaError_t cg_first(gbds_solver s, const CgFields &f, cudaStream_t st) {
+    cudaError_t e = apply_M<T>(s, f.gauge, f.recon, f.p, f.t, f.Mp, +1, s->partials, st);
+    return e == cudaSuccess ? finish_on(s, kAlpha, st, sizeof(T) == 4 ? f32_partials(s->g, f.recon) : 0) : e;
+}
+
+template <typename T>
+cudaError_t cg_second(gbds_solver s, const CgFields &f, cudaStream_t st) {
     const Geom &g = s->g;
-    const int parts = sizeof(T) == 4 ? f32_partials(g, recon) : 0;
-    auto first = [&] {
-        cudaError_t e = apply_M<T>(s, gauge, recon, p, t, Mp, +1, s->partials, st);
-        return e == cudaSuccess ? finish_on(s, kAlpha, st, parts) : e;
-    };
-    auto second = [&] {
-        cudaError_t e = apply_Mdag_update<T>(s, gauge, recon, Mp, t, r, st);
-        if (e == cudaSuccess) e = finish_on(s, kBeta, st, parts);
-        if (e != cudaSuccess) return e;
-        launch_pdl(cg_xpay<T>, dim3(blocks(g)), kThreads, st, static_cast<const SV<T> *>(r), static_cast<SV<T> *>(x),
-                   static_cast<SV<T> *>(p), (const Scalars *)s->sc, g.Vh, g.stride);
-        count_launch();
-        return cudaGetLastError();
-    };
-    return cg_loop(s, first, second, sizeof(T) == 4 ? 4 : 1, sizeof(T) == 4, target_rr, max_iter, iters, st);
+    cudaError_t e = apply_Mdag_update<T>(s, f.gauge, f.recon, f.Mp, f.t, f.r, st);
+    if (e == cudaSuccess) e = finish_on(s, kBeta, st, sizeof(T) == 4 ? f32_partials(g, f.recon) : 0);
+    if (e != cudaSuccess) return e;
+    launch_pdl(cg_xpay<T>, dim3(blocks(g)), kThreads, st, static_cast<const SV<T> *>(f.r), static_cast<SV<T> *>(f.x),
+               static_cast<SV<T> *>(f.p), (const Scalars *)s->sc, g.Vh, g.stride);
+    count_launch();
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t cg(gbds_solver s, const CgFields &f, double target_rr, int max_iter, int *iters, cudaStream_t st) {
+    constexpr bool inner = sizeof(T) == 4;
+    return cg_loop(
+        s, [&](cudaStream_t t) { return cg_first<T>(s, f, t); }, [&](cudaStream_t t) { return cg_second<T>(s, f, t); },
+        inner ? &s->steps : nullptr, inner, target_rr, max_iter, iters, st);
+}
+
+// second() and kCheck - 1 whole iterations, recorded
+template <typename FIRST, typename SECOND>
+void record_steps(gbds_solver s, const FIRST &first, const SECOND &second) {
+    record(s->steps, kCheck * kSecondLaunches + (kCheck - 1) * kFirstLaunches, [&](cudaStream_t cs) {
+        cudaError_t e = second(cs);
+        for (int i = 1; i < kCheck && e == cudaSuccess; i++) {
+            e = first(cs);
+            if (e == cudaSuccess) e = second(cs);
+        }
+        return e;
+    });
 }
 
 // The 16-bit operator: out = in - kappa^2 D_eo D_oe in, FP16 links.
@@ -542,22 +621,45 @@ cudaError_t apply_Mdag_update_h(gbds_solver s, const void *in, void *tmp, void *
 }
 
 template <int FMT>
-cudaError_t cg_h(gbds_solver s, double target_rr, int max_iter, int *iters, cudaStream_t st) {
+cudaError_t cg_first_h(gbds_solver s, cudaStream_t st) {
+    cudaError_t e = apply_M_h(s, s->p16, s->t16, s->Mp16, +1, s->partials, st);
+    return e == cudaSuccess ? finish_on(s, kAlpha, st) : e;
+}
+
+template <int FMT>
+cudaError_t cg_second_h(gbds_solver s, cudaStream_t st) {
     const Geom &g = s->g;
-    auto first = [&] {
-        cudaError_t e = apply_M_h(s, s->p16, s->t16, s->Mp16, +1, s->partials, st);
-        return e == cudaSuccess ? finish_on(s, kAlpha, st) : e;
-    };
-    auto second = [&] {
-        cudaError_t e = apply_Mdag_update_h(s, s->Mp16, s->t16, s->r32, st);
-        if (e == cudaSuccess) e = finish_on(s, kBeta, st);
-        if (e != cudaSuccess) return e;
-        launch_pdl(cg_xpay_h<FMT>, dim3(blocks(g)), kThreads, st, static_cast<const float4 *>(s->r32),
-                   static_cast<float4 *>(s->e32), static_cast<char *>(s->p16), (const Scalars *)s->sc, g.Vh, g.stride);
-        count_launch();
-        return cudaGetLastError();
-    };
-    return cg_loop(s, first, second, 4, true, target_rr, max_iter, iters, st);
+    cudaError_t e = apply_Mdag_update_h(s, s->Mp16, s->t16, s->r32, st);
+    if (e == cudaSuccess) e = finish_on(s, kBeta, st);
+    if (e != cudaSuccess) return e;
+    launch_pdl(cg_xpay_h<FMT>, dim3(blocks(g)), kThreads, st, static_cast<const float4 *>(s->r32),
+               static_cast<float4 *>(s->e32), static_cast<char *>(s->p16), (const Scalars *)s->sc, g.Vh, g.stride);
+    count_launch();
+    return cudaGetLastError();
+}
+
+template <int FMT>
+cudaError_t cg_h(gbds_solver s, double target_rr, int max_iter, int *iters, cudaStream_t st) {
+    return cg_loop(
+        s, [&](cudaStream_t t) { return cg_first_h<FMT>(s, t); }, [&](cudaStream_t t) { return cg_second_h<FMT>(s, t); },
+        &s->steps, true, target_rr, max_iter, iters, st);
+}
+
+// Record the inner CG's steps (inner_prec 32, 16 or 17).
+void record_inner(gbds_solver s) {
+    if (s->prm.inner_prec == 32) {
+        const CgFields f = inner_fields(s);
+        return record_steps(
+            s, [&](cudaStream_t t) { return cg_first<float>(s, f, t); },
+            [&](cudaStream_t t) { return cg_second<float>(s, f, t); });
+    }
+    if (s->fmt16 == kFmtF16N)
+        return record_steps(
+            s, [&](cudaStream_t t) { return cg_first_h<kFmtF16N>(s, t); },
+            [&](cudaStream_t t) { return cg_second_h<kFmtF16N>(s, t); });
+    return record_steps(
+        s, [&](cudaStream_t t) { return cg_first_h<kFmtBF16>(s, t); },
+        [&](cudaStream_t t) { return cg_second_h<kFmtBF16>(s, t); });
 }
 
 template <typename T>
@@ -585,11 +687,13 @@ void release(gbds_solver s) {
         if (b) cudaFree(b);
     if (s->hsc) cudaFreeHost(s->hsc);
     if (s->read) cudaEventDestroy(s->read);
+    if (s->steps.exec) cudaGraphExecDestroy(s->steps.exec);
 }
 
 }  // namespace
 
-extern "C" int gbds_solver_create(gbds_solver *out, const int dims[4], const gbds_solver_params *p) {
+// single: solves on its own (else the batched solver's FP64 side)
+static int create_solver(gbds_solver *out, const int dims[4], const gbds_solver_params *p, bool single) {
     if (!out || !p) return set_error(GBDS_ERROR_INVALID_VALUE, "NULL argument");
     *out = nullptr;
     if (p->inner_prec != 64 && p->inner_prec != 32 && p->inner_prec != 16 && p->inner_prec != 17)
@@ -636,6 +740,7 @@ extern "C" int gbds_solver_create(gbds_solver *out, const int dims[4], const gbd
     if (e == cudaSuccess) e = cudaMalloc(&s->sc, sizeof(Scalars));
     if (e == cudaSuccess) e = cudaMallocHost(&s->hsc, sizeof(Scalars));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->read, cudaEventDisableTiming);
+    if (e == cudaSuccess && p->inner_prec != 64 && single) record_inner(s);
     if (e != cudaSuccess) {
         release(s);
         delete s;
@@ -643,6 +748,10 @@ extern "C" int gbds_solver_create(gbds_solver *out, const int dims[4], const gbd
     }
     *out = s;
     return GBDS_SUCCESS;
+}
+
+extern "C" int gbds_solver_create(gbds_solver *out, const int dims[4], const gbds_solver_params *p) {
+    return create_solver(out, dims, p, true);
 }
 
 extern "C" int gbds_solver_destroy(gbds_solver s) {
@@ -769,8 +878,7 @@ static int solve_mixed(gbds_solver s, const double *b_packed, double *x_packed, 
         if (need > delta) delta = need;
         int it = 0;
         if (!half)
-            e = cg<float>(s, s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Mp32, s->t32,
-                          delta * delta, s->prm.max_iter - total, &it, st);
+            e = cg<float>(s, inner_fields(s), delta * delta, s->prm.max_iter - total, &it, st);
         else if (s->fmt16 == kFmtF16N)
             e = cg_h<kFmtF16N>(s, delta * delta, s->prm.max_iter - total, &it, st);
         else
@@ -837,8 +945,7 @@ static int solve_impl(gbds_solver s, const double *b_packed, double *x_packed, g
             e = norm_into<double>(s, s->c64, s->r64, s->p64, kSetRR, st);
             int it = 0;
             if (e == cudaSuccess)
-                e = cg<double>(s, s->gauge64, 18, s->x64, s->r64, s->p64, s->Mp64, s->t64, tol2 * c2,
-                               s->prm.max_iter, &it, st);
+                e = cg<double>(s, {s->gauge64, 18, s->x64, s->r64, s->p64, s->Mp64, s->t64}, tol2 * c2, s->prm.max_iter, &it, st);
             total = it;
             out.cycles = 1;
         } else {
@@ -871,8 +978,7 @@ static int solve_impl(gbds_solver s, const double *b_packed, double *x_packed, g
                 if (need > delta) delta = need;
                 int it = 0;
                 if (!half)
-                    e = cg<float>(s, s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Mp32, s->t32,
-                                  delta * delta, s->prm.max_iter - total, &it, st);
+                    e = cg<float>(s, inner_fields(s), delta * delta, s->prm.max_iter - total, &it, st);
                 else if (s->fmt16 == kFmtF16N)
                     e = cg_h<kFmtF16N>(s, delta * delta, s->prm.max_iter - total, &it, st);
                 else
@@ -1182,6 +1288,7 @@ struct gbds_bsolver_s {
     void *e = nullptr, *r = nullptr, *p = nullptr, *Ap = nullptr, *Mp = nullptr, *t = nullptr;  // multi-RHS FP32
     double *bpartials = nullptr, *bpartials2 = nullptr;
     unsigned *ticket = nullptr;  // 0 between launches of bfinish
+    IterGraph steps;             // kCheck iterations of the inner CG
     BScalars *bsc = nullptr, *hbsc = nullptr;
 };
 
@@ -1250,13 +1357,42 @@ cudaError_t read_bscalars(gbds_bsolver b, cudaStream_t st) {
     return e;
 }
 
+// One iteration of the lockstep CG (7 launches, 8 without the fused update).
+cudaError_t bcg_iteration(gbds_bsolver b, cudaStream_t st) {
+    const long long n = bcount(b);
+    const int nb = bblocks(b);
+    const size_t cs = bcs(b);
+    const int nr = b->nrhs;
+    cudaError_t e = apply_Mb(b, b->p, b->Mp, +1, b->bpartials, st);
+    if (e == cudaSuccess) e = bfinish_on(b, kBAlpha, st);
+    if (e == cudaSuccess && fused_update(b)) {
+        e = apply_Mb_dagger_update(b, b->Mp, st);
+    } else if (e == cudaSuccess) {
+        e = apply_Mb(b, b->Mp, b->Ap, -1, nullptr, st);
+        if (e != cudaSuccess) return e;
+#define GBDS_UPD(NR)                                                                                      \
+    launch_pdl(bcg_update<NR>, dim3(nb), 128, st, static_cast<float4 *>(b->r), static_cast<const float4 *>(b->Ap), \
+               (const BScalars *)b->bsc, n, cs, b->bpartials)
+        GBDS_BN(nr, GBDS_UPD)
+#undef GBDS_UPD
+        count_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = bfinish_on(b, kBBeta, st);
+    if (e != cudaSuccess) return e;
+#define GBDS_XP(NR)                                                                                         \
+    launch_pdl(bcg_xpay<NR>, dim3(nb), 128, st, static_cast<float4 *>(b->e), static_cast<const float4 *>(b->r), \
+               static_cast<float4 *>(b->p), (const BScalars *)b->bsc, n, cs)
+    GBDS_BN(nr, GBDS_XP)
+#undef GBDS_XP
+    count_launch();
+    return cudaGetLastError();
+}
+
 // Lockstep CG on the active right-hand sides (x = e = 0, r = p = residual,
 // rr set); each stops at rr <= target[q] or when it stagnates.
 cudaError_t bcg(gbds_bsolver b, const std::vector<double> &target, int max_iter, std::vector<int> &iters,
                 cudaStream_t st) {
-    const long long n = bcount(b);
-    const int nb = bblocks(b);
-    const size_t cs = bcs(b);
     const int nr = b->nrhs;
     std::vector<double> best(nr, 1e300);
     std::vector<int> best_k(nr, 0);
@@ -1266,37 +1402,18 @@ cudaError_t bcg(gbds_bsolver b, const std::vector<double> &target, int max_iter,
         bool any = false;
         for (int q = 0; q < nr; q++) any |= b->hbsc[q].active != 0;
         if (!any) break;
-        e = apply_Mb(b, b->p, b->Mp, +1, b->bpartials, st);
-        if (e == cudaSuccess) e = bfinish_on(b, kBAlpha, st);
-        if (e == cudaSuccess && fused_update(b)) {
-            e = apply_Mb_dagger_update(b, b->Mp, st);
-        } else if (e == cudaSuccess) {
-            e = apply_Mb(b, b->Mp, b->Ap, -1, nullptr, st);
-        }
-        if (e == cudaSuccess && !fused_update(b)) {
-#define GBDS_UPD(NR)                                                                                      \
-    launch_pdl(bcg_update<NR>, dim3(nb), 128, st, static_cast<float4 *>(b->r), static_cast<const float4 *>(b->Ap), \
-               (const BScalars *)b->bsc, n, cs, b->bpartials)
-            GBDS_BN(nr, GBDS_UPD)
-#undef GBDS_UPD
-            count_launch();
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = bfinish_on(b, kBBeta, st);
-        if (e == cudaSuccess) {
-#define GBDS_XP(NR)                                                                                         \
-    launch_pdl(bcg_xpay<NR>, dim3(nb), 128, st, static_cast<float4 *>(b->e), static_cast<const float4 *>(b->r), \
-               static_cast<float4 *>(b->p), (const BScalars *)b->bsc, n, cs)
-            GBDS_BN(nr, GBDS_XP)
-#undef GBDS_XP
-            count_launch();
-            e = cudaGetLastError();
+        int done = 1;
+        if (b->steps.exec && k % kCheck == 0 && k + kCheck <= max_iter) {
+            e = launch(b->steps, st);
+            done = kCheck;
+        } else {
+            e = bcg_iteration(b, st);
         }
         if (e != cudaSuccess) break;
-        k++;
+        k += done;
         for (int q = 0; q < nr; q++)
-            if (b->hbsc[q].active) iters[q]++;
-        if (k % 4 == 0 || k == max_iter) {
+            if (b->hbsc[q].active) iters[q] += done;
+        if (k % kCheck == 0 || k == max_iter) {
             e = read_bscalars(b, st);
             if (e != cudaSuccess) break;
             bool changed = false;
@@ -1325,6 +1442,7 @@ void brelease(gbds_bsolver b) {
     for (void *p : bufs)
         if (p) cudaFree(p);
     if (b->hbsc) cudaFreeHost(b->hbsc);
+    if (b->steps.exec) cudaGraphExecDestroy(b->steps.exec);
     if (b->s1) gbds_solver_destroy(b->s1);
 }
 
@@ -1339,7 +1457,7 @@ extern "C" int gbds_bsolver_create(gbds_bsolver *out, const int dims[4], int nrh
     gbds_bsolver b = new (std::nothrow) gbds_bsolver_s;
     if (!b) return set_error(GBDS_ERROR_OUT_OF_MEMORY, "host allocation failed");
     b->nrhs = nrhs;
-    int rc = gbds_solver_create(&b->s1, dims, p);
+    int rc = create_solver(&b->s1, dims, p, false);
     if (rc != GBDS_SUCCESS) {
         delete b;
         return rc;
@@ -1364,6 +1482,12 @@ extern "C" int gbds_bsolver_create(gbds_bsolver *out, const int dims[4], int nrh
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // zero for every stream
     if (e == cudaSuccess) e = cudaMalloc(&b->bsc, sizeof(BScalars) * nrhs);
     if (e == cudaSuccess) e = cudaMallocHost(&b->hbsc, sizeof(BScalars) * nrhs);
+    if (e == cudaSuccess)
+        record(b->steps, kCheck * (fused_update(b) ? 7 : 8), [&](cudaStream_t cs) {
+            cudaError_t le = cudaSuccess;
+            for (int i = 0; i < kCheck && le == cudaSuccess; i++) le = bcg_iteration(b, cs);
+            return le;
+        });
     if (e != cudaSuccess) {
         brelease(b);
         delete b;
