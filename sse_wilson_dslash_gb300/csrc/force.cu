@@ -140,13 +140,11 @@ struct ForceArgs {
     int accumulate;
 };
 
-// Sites per CTA: 128 in FP32, 64 in FP64, so that the staged output of a CTA
-// (2 links x 18 reals per site at a time) is 18 KB of shared memory either
-// way; FP32 caps registers for 7 CTAs per SM.
-template <typename T> struct ForceTile {
-    static constexpr int sites = sizeof(T) == 4 ? 128 : 64;
-    static constexpr int min_blocks = sizeof(T) == 4 ? 7 : 1;
-};
+// Sites per CTA; stage of their links' output in shared memory, a site every
+// stage_pitch reals: two (FP32) or one (FP64) more than its 72, so that the 8-byte
+// stores of a half-warp's sites fall into different banks.
+constexpr int kForceSites = 32;
+template <typename T> constexpr int stage_pitch() { return sizeof(T) == 4 ? 74 : 73; }
 
 // R = G (mode 0) or TA(G U^+) (mode 1) of link (p, h, MU), times coef, into
 // o[(3j+i)*2 + 0/1] = R_ij: the packed transposed order of the output.
@@ -197,83 +195,74 @@ __device__ __forceinline__ void force_link(const ForceArgs &a, int p, int h, con
     for (int j = 0; j < 3; j++)
 #pragma unroll
         for (int i = 0; i < 3; i++) {
-            o[(j * 3 + i) * 2] = c * R[i][j].r;
-            o[(j * 3 + i) * 2 + 1] = c * R[i][j].i;
+            if constexpr (sizeof(T) == 4) {
+                *reinterpret_cast<float2 *>(o + (j * 3 + i) * 2) = make_float2(c * R[i][j].r, c * R[i][j].i);
+            } else {
+                o[(j * 3 + i) * 2] = c * R[i][j].r;
+                o[(j * 3 + i) * 2 + 1] = c * R[i][j].i;
+            }
         }
 }
 
-// One thread per site of checkerboard p = blockIdx.y (both checkerboards in
-// one launch; they own disjoint links), all four links of the site.  The
-// site's own spinor (chi on checkerboard pt, psi on cb) is loaded once for
-// the four links.  The results go out in two halves (links 0-1, then 2-3),
-// each staged in shared memory and written with 16-byte stores: in the
-// canonical layout a CTA's sites are one contiguous run of the packed output
-// and each half a 36-real block per site; with a caller layout each warp
-// writes its sites' blocks one site at a time.
-template <typename T, int ISIGN, int HALF>
-__device__ __forceinline__ void force_half(const ForceArgs &a, int p, int h0, int h, const Nbr &n,
-                                           const cx<T> (&own)[4][3], T *stage) {
+// A CTA takes 32 sites of one checkerboard (even and odd CTAs alternate, so that
+// a spinor's use as a site's own and as its neighbours' meet in L2; they own
+// disjoint links), warp mu their links mu, so that a thread's
+// loads (the site's own spinor, chi on checkerboard pt, psi on cb; one
+// neighbour's; the link) are all in flight at once.  The 72-real blocks of the
+// sites are staged in shared memory and written with 16-byte stores: in the
+// canonical layout one contiguous run of the packed output, with a caller
+// layout site by site.  Bound by DRAM and the latency of its loads: 32^3x64 FP32
+// 286 -> 251 us (0.84 of the HBM floor of 211) against one thread a site that
+// took the four links in turn and wrote each site's block in two 144-byte
+// halves.  Registers capped for 36 warps per SM: 274 us at 28, 261 at 32, 280 at
+// 40; links marked for early eviction 254.
+template <typename T, int ISIGN>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 9 : 1) force_kernel(const ForceArgs a) {
+    using F = Field<T>;
     using Q = typename VecOf<T>::S;  // 16-byte vector: float4 or double2
-    constexpr int NS = ForceTile<T>::sites;
-    constexpr int QPS = 72 * (int)sizeof(T) / 16;  // 16-byte vectors per site
-    constexpr int QH = QPS / 2;                    // per half
+    constexpr int PITCH = stage_pitch<T>(), QN = 16 / (int)sizeof(T);
+    constexpr int QPS = 72 / QN;  // 16-byte vectors per site
+    __shared__ __align__(16) T stage[kForceSites * PITCH];
+    const int p = blockIdx.x & 1;
+    const int h0 = (blockIdx.x >> 1) * kForceSites;
+    const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+    const int h = h0 + lane;
     if (h < a.g.Vh) {
-        T *st = stage + threadIdx.x * 36;
-        force_link<T, ISIGN, 2 * HALF>(a, p, h, n, own, st);
-        force_link<T, ISIGN, 2 * HALF + 1>(a, p, h, n, own, st + 18);
+        Nbr n;
+        cx<T> own[4][3];
+        neighbours<4>(a.g, h, p, n);
+        F::load_spinor(static_cast<const Q *>(p == a.pt ? a.chi : a.psi), a.g.stride, h, own);
+        T *st = stage + lane * PITCH + mu * 18;
+        if (mu == 0) force_link<T, ISIGN, 0>(a, p, h, n, own, st);
+        else if (mu == 1) force_link<T, ISIGN, 1>(a, p, h, n, own, st);
+        else if (mu == 2) force_link<T, ISIGN, 2>(a, p, h, n, own, st);
+        else force_link<T, ISIGN, 3>(a, p, h, n, own, st);
     }
     __syncthreads();
-    const int nsites = min(NS, a.g.Vh - h0);
-    const Q *sq = reinterpret_cast<const Q *>(stage);
+    const int nsites = min(kForceSites, a.g.Vh - h0);
     Q *out = static_cast<Q *>(a.out);
-    if (!a.table) {
-        Q *dst = out + (size_t)(p * a.g.Vh + h0) * QPS + HALF * QH;
-        for (int i = threadIdx.x; i < nsites * QH; i += NS) {
-            const int s = i / QH, j = i - s * QH;
-            Q v = sq[i];
-            Q *d = dst + (size_t)s * QPS + j;
+    for (int i = threadIdx.x; i < nsites * QPS; i += 128) {
+        const int s = i / QPS, j = i - s * QPS;
+        const size_t site = a.table ? (size_t)a.table[p * a.g.Vh + h0 + s] : (size_t)p * a.g.Vh + h0 + s;
+        const T *v = stage + s * PITCH + j * QN;
+        Q *d = out + site * QPS + j;
+        if constexpr (sizeof(T) == 4) {
+            const float2 lo = *reinterpret_cast<const float2 *>(v), hi = *reinterpret_cast<const float2 *>(v + 2);
+            float4 q = make_float4(lo.x, lo.y, hi.x, hi.y);
             if (a.accumulate) {
-                const Q w = *d;
-                if constexpr (sizeof(T) == 4) v = make_float4(w.x + v.x, w.y + v.y, w.z + v.z, w.w + v.w);
-                else v = make_double2(w.x + v.x, w.y + v.y);
+                const float4 w = *d;
+                q = make_float4(w.x + q.x, w.y + q.y, w.z + q.z, w.w + q.w);
             }
-            *d = v;
-        }
-    } else {
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        for (int k = w * 32; k < min(nsites, w * 32 + 32); k++) {
-            Q *dst = out + (size_t)a.table[p * a.g.Vh + h0 + k] * QPS + HALF * QH;
-            for (int i = lane; i < QH; i += 32) {
-                Q v = sq[k * QH + i];
-                if (a.accumulate) {
-                    const Q w2 = dst[i];
-                    if constexpr (sizeof(T) == 4) v = make_float4(w2.x + v.x, w2.y + v.y, w2.z + v.z, w2.w + v.w);
-                    else v = make_double2(w2.x + v.x, w2.y + v.y);
-                }
-                dst[i] = v;
+            __stcs(d, q);
+        } else {
+            double2 q = make_double2(v[0], v[1]);
+            if (a.accumulate) {
+                const double2 w = *d;
+                q = make_double2(w.x + q.x, w.y + q.y);
             }
+            __stcs(d, q);
         }
     }
-    __syncthreads();  // the staging area is refilled by the next half
-}
-
-template <typename T, int ISIGN>
-__global__ void __launch_bounds__(ForceTile<T>::sites, ForceTile<T>::min_blocks) force_kernel(const ForceArgs a) {
-    using F = Field<T>;
-    using V = typename VecOf<T>::S;
-    constexpr int NS = ForceTile<T>::sites;
-    __shared__ __align__(16) T stage[NS * 36];
-    const int p = blockIdx.y;
-    const int h0 = blockIdx.x * NS;
-    const int h = h0 + threadIdx.x;
-    Nbr n;
-    cx<T> own[4][3];
-    if (h < a.g.Vh) {
-        neighbours<4>(a.g, h, p, n);
-        F::load_spinor(static_cast<const V *>(p == a.pt ? a.chi : a.psi), a.g.stride, h, own);
-    }
-    force_half<T, ISIGN, 0>(a, p, h0, h, n, own, stage);
-    force_half<T, ISIGN, 1>(a, p, h0, h, n, own, stage);
 }
 
 }  // namespace
@@ -305,16 +294,13 @@ extern "C" int gbds_op_force(gbds_op op, const void *gauge, const void *psi, con
     if ((reinterpret_cast<uintptr_t>(force_packed) & 15u) != 0)
         return set_error(GBDS_ERROR_INVALID_VALUE, "force_packed must be 16-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const dim3 grid(2 * ((op->g.Vh + kForceSites - 1) / kForceSites));
     if (op->prec == 32) {
-        constexpr int ns = ForceTile<float>::sites;
-        const dim3 grid((op->g.Vh + ns - 1) / ns, 2);
-        if (isign > 0) force_kernel<float, 1><<<grid, ns, 0, st>>>(a);
-        else force_kernel<float, -1><<<grid, ns, 0, st>>>(a);
+        if (isign > 0) force_kernel<float, 1><<<grid, 128, 0, st>>>(a);
+        else force_kernel<float, -1><<<grid, 128, 0, st>>>(a);
     } else {
-        constexpr int ns = ForceTile<double>::sites;
-        const dim3 grid((op->g.Vh + ns - 1) / ns, 2);
-        if (isign > 0) force_kernel<double, 1><<<grid, ns, 0, st>>>(a);
-        else force_kernel<double, -1><<<grid, ns, 0, st>>>(a);
+        if (isign > 0) force_kernel<double, 1><<<grid, 128, 0, st>>>(a);
+        else force_kernel<double, -1><<<grid, 128, 0, st>>>(a);
     }
     count_launch();
     cudaError_t e = cudaGetLastError();
