@@ -6,10 +6,10 @@ namespace {
 
 template <int ND, int RECON, int EPI = 0>
 cudaError_t launch_split(const DslashArgs<float> &a, int isign, cudaStream_t st, const float4 *x = nullptr, float coef = 0.f,
-                         const CgUpdate<float> &upd = {}, double *partials = nullptr) {
+                         const CgUpdate<float> &upd = {}, double *partials = nullptr, const SumHere &here = {}) {
     const dim3 grid((a.g.Vh + kSplitSites - 1) / kSplitSites);
-    if (isign > 0) launch_pdl(dslash_split_kernel<ND, RECON, 1, EPI>, grid, 128, st, a, x, coef, upd, partials);
-    else launch_pdl(dslash_split_kernel<ND, RECON, -1, EPI>, grid, 128, st, a, x, coef, upd, partials);
+    if (isign > 0) launch_pdl(dslash_split_kernel<ND, RECON, 1, EPI>, grid, 128, st, a, x, coef, upd, partials, here);
+    else launch_pdl(dslash_split_kernel<ND, RECON, -1, EPI>, grid, 128, st, a, x, coef, upd, partials, here);
     count_launch();
     return cudaGetLastError();
 }
@@ -78,18 +78,20 @@ namespace {
 
 template <bool UPD>
 cudaError_t launch_epilogue(const Geom &g, int recon, const void *gauge, const void *psi, const void *x, float coef, void *res,
-                            double *partials, int isign, int cb, cudaStream_t st, const CgUpdate<float> &upd = {}) {
+                            double *partials, int isign, int cb, cudaStream_t st, const SumHere &here,
+                            const CgUpdate<float> &upd = {}) {
     int block, variant;
     f32_tuning(g, recon, &block, &variant);
     constexpr int EPI = UPD ? 2 : 1;
     if (variant == kSplitVariant) {
         const DslashArgs<float> a = f32_args(g, recon, gauge, psi, res, cb);
         const float4 *xv = static_cast<const float4 *>(x);
-        return recon == 18 ? launch_split<4, 18, EPI>(a, isign, st, xv, coef, upd, partials)
-                           : launch_split<4, 12, EPI>(a, isign, st, xv, coef, upd, partials);
+        return recon == 18 ? launch_split<4, 18, EPI>(a, isign, st, xv, coef, upd, partials, here)
+                           : launch_split<4, 12, EPI>(a, isign, st, xv, coef, upd, partials, here);
     }
     if (variant == 0)
-        return launch_dslash_xpay_t<float, UPD, 0, 0>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st, upd);
+        return launch_dslash_xpay_t<float, UPD, 0, 0>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st, upd,
+                                                      here);
     return launch_dslash_xpay_t<float, UPD>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st, upd);
 }
 
@@ -101,14 +103,21 @@ int f32_partials(const Geom &g, int recon) {
     return variant == kSplitVariant ? (g.Vh + kSplitSites - 1) / kSplitSites : xpay_blocks(g);
 }
 
+bool f32_sums_here(const Geom &g, int recon) {
+    int block, variant;
+    f32_tuning(g, recon, &block, &variant);
+    return variant == kSplitVariant || (variant == 0 && xpay_blocks(g) <= 512);
+}
+
 cudaError_t launch_dslash_xpay_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
-                                   float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream) {
-    return launch_epilogue<false>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, stream);
+                                   float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream,
+                                   const SumHere &here) {
+    return launch_epilogue<false>(g, recon, gauge, psi, x, coef, res, partials, isign, cb, stream, here);
 }
 cudaError_t launch_dslash_cg_update_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
                                         float coef, const double *alpha, void *r, double *partials, int isign, int cb,
-                                        cudaStream_t stream) {
-    return launch_epilogue<true>(g, recon, gauge, psi, x, coef, nullptr, partials, isign, cb, stream,
+                                        cudaStream_t stream, const SumHere &here) {
+    return launch_epilogue<true>(g, recon, gauge, psi, x, coef, nullptr, partials, isign, cb, stream, here,
                                  {static_cast<float4 *>(r), alpha});
 }
 }  // namespace gbds

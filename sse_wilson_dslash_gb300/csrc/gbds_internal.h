@@ -46,17 +46,38 @@ cudaError_t launch_dslash_f64(const Geom &g, int recon, const void *gauge, const
 // variant indices the tuning calls accept (FP64: three, all the same kernel)
 int dslash_variants(int prec);
 
+// Scalars of a CG (device).
+struct CgScalars {
+    double rr;        // |r|^2 of the running CG
+    double pAp;       // <p, A p> = |M p|^2
+    double alpha, beta;
+    double outer_rr;  // |r|^2 of the FP64 defect-correction residual
+    double norm;      // scratch result of a norm
+};
+// What a sum is for.
+enum FinishMode { kAlpha = 0, kBeta = 1, kSetRR = 2, kOuterRR = 3, kNorm = 4 };
+// A launch that finishes its sum itself (f32_sums_here): ticket is 0 between
+// launches.
+struct SumHere {
+    unsigned *ticket = nullptr;
+    CgScalars *sc = nullptr;
+    int mode = kNorm;
+};
+
 // res = x + coef * Dslash(psi) (4D; res and x on checkerboard 1-cb); if
 // partials != nullptr, partials[b] = sum of |res|^2 over launch block b (there
 // are (Vh + 127) / 128 blocks; FP32: f32_partials).
 int f32_partials(const Geom &g, int recon);
+// whether the FP32 launches take `here` (else the caller adds the partials up)
+bool f32_sums_here(const Geom &g, int recon);
 cudaError_t launch_dslash_xpay_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
-                                   float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream);
+                                   float coef, void *res, double *partials, int isign, int cb, cudaStream_t stream,
+                                   const SumHere &here = {});
 // r -= alpha (x + coef * Dslash(psi)), alpha read on the device, with |r|^2 in
 // the partials (as above)
 cudaError_t launch_dslash_cg_update_f32(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
                                         float coef, const double *alpha, void *r, double *partials, int isign, int cb,
-                                        cudaStream_t stream);
+                                        cudaStream_t stream, const SumHere &here = {});
 // (18-real links)
 cudaError_t launch_dslash_cg_update_f64(const Geom &g, const void *gauge, const void *psi, const void *x, double coef,
                                         const double *alpha, void *r, double *partials, int isign, int cb,

@@ -35,13 +35,7 @@
 namespace gbds {
 namespace {
 
-struct Scalars {
-    double rr;        // |r|^2 of the running CG
-    double pAp;       // <p, A p> = |M p|^2
-    double alpha, beta;
-    double outer_rr;  // |r|^2 of the FP64 defect-correction residual
-    double norm;      // scratch result of a norm
-};
+using Scalars = CgScalars;
 
 constexpr int kThreads = 128;
 
@@ -287,8 +281,6 @@ __global__ void __launch_bounds__(kThreads) scale_copy_h(const float4 *__restric
     Sio<FMT>::store(p, stride, h, ps);
 }
 
-enum FinishMode { kAlpha = 0, kBeta = 1, kSetRR = 2, kOuterRR = 3, kNorm = 4 };
-
 // Deterministic sum of the block partials (fixed order), then the scalar step.
 __global__ void __launch_bounds__(1024) finish(const double *partials, int n, Scalars *sc, int mode) {
     pdl_allow_next();
@@ -303,14 +295,7 @@ __global__ void __launch_bounds__(1024) finish(const double *partials, int n, Sc
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
-    const double sum = buf[0];
-    switch (mode) {
-    case kAlpha: sc->pAp = sum; sc->alpha = sum > 0 ? sc->rr / sum : 0.0; break;
-    case kBeta: sc->beta = sc->rr > 0 ? sum / sc->rr : 0.0; sc->rr = sum; break;
-    case kSetRR: sc->rr = sum; break;
-    case kOuterRR: sc->outer_rr = sum; break;
-    default: sc->norm = sum; break;
-    }
+    sum_step(sc, mode, buf[0]);
 }
 
 __global__ void f64_to_f32(const double *__restrict__ a, float *b, size_t n) {
@@ -356,6 +341,7 @@ struct gbds_solver_s {
     Scalars *hsc = nullptr;   // pinned host copy
     cudaEvent_t read = nullptr;  // the copy of a convergence test has arrived
     IterGraph steps;             // the inner CG's
+    unsigned *ticket = nullptr;  // 0 between launches (SumHere)
     bool have_gauge = false;
 };
 
@@ -375,8 +361,9 @@ cudaError_t dslash(const Geom &g, int recon, const void *gauge, const void *psi,
 
 template <typename T>
 cudaError_t dslash_xpay(const Geom &g, int recon, const void *gauge, const void *psi, const void *x, T coef, void *res,
-                        double *partials, int isign, int cb, cudaStream_t st) {
-    if constexpr (sizeof(T) == 4) return launch_dslash_xpay_f32(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st);
+                        double *partials, int isign, int cb, cudaStream_t st, const SumHere &here) {
+    if constexpr (sizeof(T) == 4)
+        return launch_dslash_xpay_f32(g, recon, gauge, psi, x, coef, res, partials, isign, cb, st, here);
     else return launch_dslash_xpay_f64(g, gauge, psi, x, coef, res, partials, isign, cb, st);
 }
 
@@ -390,25 +377,26 @@ cudaError_t finish_on(gbds_solver s, int mode, cudaStream_t st, int n = 0) {
 // out_e = in_e - kappa^2 D_eo(isign) D_oe(isign) in_e  (partials: |out|^2)
 template <typename T>
 cudaError_t apply_M(gbds_solver s, const void *gauge, int recon, const void *in, void *tmp, void *out, int isign,
-                    double *partials, cudaStream_t st) {
+                    double *partials, cudaStream_t st, const SumHere &here = {}) {
     const Geom &g = s->g;
     const double k2 = s->prm.kappa * s->prm.kappa;
     cudaError_t e = dslash<T>(g, recon, gauge, in, tmp, isign, 0, st);
     if (e != cudaSuccess) return e;
-    return dslash_xpay<T>(g, recon, gauge, tmp, in, (T)(-k2), out, partials, isign, 1, st);
+    return dslash_xpay<T>(g, recon, gauge, tmp, in, (T)(-k2), out, partials, isign, 1, st, here);
 }
 
 // r -= alpha M^+ in, |r|^2 in the partials: M^+'s second launch updates r in
 // place of storing M^+ in
 template <typename T>
 cudaError_t apply_Mdag_update(gbds_solver s, const void *gauge, int recon, const void *in, void *tmp, void *r,
-                              cudaStream_t st) {
+                              cudaStream_t st, const SumHere &here) {
     const Geom &g = s->g;
     const double k2 = s->prm.kappa * s->prm.kappa;
     cudaError_t e = dslash<T>(g, recon, gauge, in, tmp, -1, 0, st);
     if (e != cudaSuccess) return e;
     if constexpr (sizeof(T) == 4)
-        return launch_dslash_cg_update_f32(g, recon, gauge, tmp, in, (float)(-k2), &s->sc->alpha, r, s->partials, -1, 1, st);
+        return launch_dslash_cg_update_f32(g, recon, gauge, tmp, in, (float)(-k2), &s->sc->alpha, r, s->partials, -1, 1, st,
+                                           here);
     else return launch_dslash_cg_update_f64(g, gauge, tmp, in, -k2, &s->sc->alpha, r, s->partials, -1, 1, st);
 }
 
@@ -561,19 +549,32 @@ CgFields inner_fields(gbds_solver s) {
     return {s->gauge32, s->prm.inner_recon, s->e32, s->r32, s->p32, s->Mp32, s->t32};
 }
 
-constexpr int kFirstLaunches = 3, kSecondLaunches = 4;  // of cg_first and cg_second
+// Whether the inner CG's operator launches finish their sums themselves (small
+// lattices), without a launch of their own.
+bool sums_here(gbds_solver s) { return s->prm.inner_prec == 32 && f32_sums_here(s->g, s->prm.inner_recon); }
+
+template <typename T>
+SumHere sum_here_to(gbds_solver s, int mode) {
+    SumHere h;
+    if (sizeof(T) == 4 && sums_here(s)) h = {s->ticket, s->sc, mode};
+    return h;
+}
 
 template <typename T>
 cudaError_t cg_first(gbds_solver s, const CgFields &f, cudaStream_t st) {
-    cudaError_t e = apply_M<T>(s, f.gauge, f.recon, f.p, f.t, f.Mp, +1, s->partials, st);
-    return e == cudaSuccess ? finish_on(s, kAlpha, st, sizeof(T) == 4 ? f32_partials(s->g, f.recon) : 0) : e;
+    const SumHere here = sum_here_to<T>(s, kAlpha);
+    cudaError_t e = apply_M<T>(s, f.gauge, f.recon, f.p, f.t, f.Mp, +1, s->partials, st, here);
+    if (e != cudaSuccess || here.ticket) return e;
+    return finish_on(s, kAlpha, st, sizeof(T) == 4 ? f32_partials(s->g, f.recon) : 0);
 }
 
 template <typename T>
 cudaError_t cg_second(gbds_solver s, const CgFields &f, cudaStream_t st) {
     const Geom &g = s->g;
-    cudaError_t e = apply_Mdag_update<T>(s, f.gauge, f.recon, f.Mp, f.t, f.r, st);
-    if (e == cudaSuccess) e = finish_on(s, kBeta, st, sizeof(T) == 4 ? f32_partials(g, f.recon) : 0);
+    const SumHere here = sum_here_to<T>(s, kBeta);
+    cudaError_t e = apply_Mdag_update<T>(s, f.gauge, f.recon, f.Mp, f.t, f.r, st, here);
+    if (e == cudaSuccess && !here.ticket)
+        e = finish_on(s, kBeta, st, sizeof(T) == 4 ? f32_partials(g, f.recon) : 0);
     if (e != cudaSuccess) return e;
     launch_pdl(cg_xpay<T>, dim3(blocks(g)), kThreads, st, static_cast<const SV<T> *>(f.r), static_cast<SV<T> *>(f.x),
                static_cast<SV<T> *>(f.p), (const Scalars *)s->sc, g.Vh, g.stride);
@@ -592,7 +593,8 @@ cudaError_t cg(gbds_solver s, const CgFields &f, double target_rr, int max_iter,
 // second() and kCheck - 1 whole iterations, recorded
 template <typename FIRST, typename SECOND>
 void record_steps(gbds_solver s, const FIRST &first, const SECOND &second) {
-    record(s->steps, kCheck * kSecondLaunches + (kCheck - 1) * kFirstLaunches, [&](cudaStream_t cs) {
+    const int n1 = sums_here(s) ? 2 : 3, n2 = sums_here(s) ? 3 : 4;  // launches of first(), second()
+    record(s->steps, kCheck * n2 + (kCheck - 1) * n1, [&](cudaStream_t cs) {
         cudaError_t e = second(cs);
         for (int i = 1; i < kCheck && e == cudaSuccess; i++) {
             e = first(cs);
@@ -682,7 +684,7 @@ void release(gbds_solver s) {
     void *bufs[] = {s->gauge64, s->gauge32, s->gauge_df, s->xdf, s->b64, s->c64, s->x64, s->r64, s->p64, s->Ap64,
                     s->Mp64, s->t64,
                     s->e32, s->r32, s->p32, s->Mp32, s->t32, s->p16, s->Mp16, s->t16, s->gauge16,
-                    s->partials, s->sc};
+                    s->partials, s->sc, s->ticket};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (s->hsc) cudaFreeHost(s->hsc);
@@ -738,6 +740,9 @@ static int create_solver(gbds_solver *out, const int dims[4], const gbds_solver_
     const int parts = std::max(blocks(g), f32_partials(g, p->inner_recon));
     if (e == cudaSuccess) e = cudaMalloc(&s->partials, sizeof(double) * (size_t)parts);
     if (e == cudaSuccess) e = cudaMalloc(&s->sc, sizeof(Scalars));
+    if (e == cudaSuccess) e = cudaMalloc(&s->ticket, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(s->ticket, 0, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // zero for every stream
     if (e == cudaSuccess) e = cudaMallocHost(&s->hsc, sizeof(Scalars));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->read, cudaEventDisableTiming);
     if (e == cudaSuccess && p->inner_prec != 64 && single) record_inner(s);
