@@ -230,6 +230,7 @@ struct GenArgs {
     // per-(block, rhs) |r|^2 partials
     const RhsCgScalars *rsc;
     float4 *rvec;
+    int reverse;  // gen_block
     const double *alpha;  // the same for nrhs 1 (16-bit storage, rvec an FP32 field)
 };
 
@@ -623,6 +624,12 @@ __device__ __forceinline__ void stage_links(const GenArgs &a, const Nbr &n, int 
     }
 }
 
+// The block's place in the lattice: from the end with a.reverse (FP32 pairs).
+template <int FMT>
+__device__ __forceinline__ int gen_block(const GenArgs &a) {
+    return FMT == kFmtF32Pairs && a.reverse ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+}
+
 // Shared memory of the staged links, (Mr, Mi) of 8 links a site: SITES sites,
 // or (0) as many as the launch gave.
 template <int SITES>
@@ -655,7 +662,7 @@ __global__ void __launch_bounds__(128, FMT == kFmtF16N && NRHS ? 5 : 7) dslash_g
     float2 (*sL)[8][9] = staged_links<NRHS ? 128 / (NRHS ? NRHS : 1) : 0>();
     const int t = threadIdx.x;
     const int p = t / nr, r = t % nr;
-    const int h = gen_site(a.g, blockIdx.x * P + p);
+    const int h = gen_site(a.g, gen_block<FMT>(a) * P + p);
     const bool act = h < a.g.Vh && (NRHS || p < P);
     if constexpr (EPI >= 2 && FMT == kFmtF32Pairs) {
         // the epilogue's operands (x, and r for the CG update) toward L2 now:
@@ -845,7 +852,7 @@ __global__ void __launch_bounds__(128, 4) dslash_gen4_kernel(const GenArgs a) {
     __shared__ float2 sL[P][8][9];  // (Mr, Mi) splats
     const int t = threadIdx.x;
     const int p = t / H, r = t % H;  // this thread: rhs r and r + H of site p
-    const int h = gen_site(a.g, blockIdx.x * P + p);
+    const int h = gen_site(a.g, gen_block<FMT>(a) * P + p);
     const bool act = h < a.g.Vh;
     Nbr n;
     if (act) neighbours<4>(a.g, h, a.pt, n);

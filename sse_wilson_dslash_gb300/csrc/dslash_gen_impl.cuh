@@ -168,8 +168,10 @@ void launch_gen5_nrhs(const GenArgs &a, int nrhs, cudaStream_t st) {
 
 template <int FMT>
 cudaError_t launch_gen_t(const Geom &g, int recon, int nrhs, const void *gauge, const void *psi, void *res, int isign,
-                         int cb, const void *x, float coef, double *partials, cudaStream_t st, int variant = 0) {
+                         int cb, const void *x, float coef, double *partials, cudaStream_t st, int variant = 0,
+                         bool reverse = false) {
     GenArgs a;
+    a.reverse = reverse;
     a.g = g;
     a.psi = static_cast<const char *>(psi);
     a.res = static_cast<char *>(res);
@@ -248,9 +250,10 @@ cudaError_t launch_gen_t(const Geom &g, int recon, int nrhs, const void *gauge, 
 template <int FMT>
 cudaError_t launch_gen_cg_update_t(const Geom &g, int recon, int nrhs, const void *gauge, const void *psi, int isign,
                                    int cb, const void *x, float coef, const RhsCgScalars *rsc, void *r, double *partials,
-                                   cudaStream_t st) {
+                                   cudaStream_t st, bool reverse) {
     if (nrhs != 8 && nrhs != 16 && nrhs != 32) return cudaErrorInvalidValue;
     GenArgs a;
+    a.reverse = reverse;
     a.g = g;
     a.psi = static_cast<const char *>(psi);
     a.res = nullptr;

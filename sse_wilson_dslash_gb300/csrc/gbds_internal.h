@@ -114,8 +114,13 @@ cudaError_t launch_pack_gauge(const Geom &g, int prec, int recon, const void *u_
 // 1, 2, 3): the whole hop in packed FP32x2 (nrhs 8, 16, 32).
 cudaError_t launch_gen_f32(const Geom &g, int recon, int nrhs, const void *gauge, const void *psi, void *res, int isign,
                            int cb, const void *x, float coef, double *partials, cudaStream_t st, int variant = 0);
+// reverse (FP32 pairs, packed kernels): the blocks go through the lattice from
+// its end.  The batched CG's launches each read what the one before wrote; in
+// alternating directions a launch starts on what is still in L2 (fields of 100 MB
+// at 16 rhs on 16^3x32, L2 129 MB): 37.9 -> 37.1 ms a solve, 8 rhs 22.0 -> 21.3.
 cudaError_t launch_gen_f32p(const Geom &g, int recon, int nrhs, const void *gauge, const void *psi, void *res, int isign,
-                            int cb, const void *x, float coef, double *partials, cudaStream_t st, int variant = 0);
+                            int cb, const void *x, float coef, double *partials, cudaStream_t st, int variant = 0,
+                            bool reverse = false);
 cudaError_t launch_gen_half(int fmt, const Geom &g, int recon, int nrhs, const void *gauge, const void *psi, void *res,
                             int isign, int cb, const void *x, float coef, double *partials, cudaStream_t st, int variant = 0);
 // packed: FP32 [nrhs][V][4][3][2], caller order
@@ -137,7 +142,7 @@ cudaError_t launch_unpack_gen_half(int fmt, const Geom &g, int nrhs, const void 
 struct RhsCgScalars;
 cudaError_t launch_gen_f32p_cg_update(const Geom &g, int recon, int nrhs, const void *gauge, const void *psi, int isign,
                                       int cb, const void *x, float coef, const RhsCgScalars *rsc, void *r,
-                                      double *partials, cudaStream_t st);
+                                      double *partials, cudaStream_t st, bool reverse = false);
 inline int gen_spinor_bytes(int fmt) { return (fmt == 0 || fmt == 3) ? 96 : (fmt == 1 ? 48 : 52); }
 // z slab of the multi-RHS kernels' site order for nrhs right-hand sides in
 // format fmt with recon-real FP32 links (0: the natural order)

@@ -1103,10 +1103,11 @@ __global__ void __launch_bounds__(128) bcg_update(float4 *r, const float4 *__res
 // x += alpha_r p;  p = r + beta_r p  (active rhs only)
 template <int NRHS>
 __global__ void __launch_bounds__(128) bcg_xpay(float4 *x, const float4 *__restrict__ r, float4 *p, const BScalars *sc,
-                                               long long n, size_t cs) {
+                                               long long n, size_t cs, int reverse) {
     pdl_allow_next();
     pdl_wait_prev();
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned block = reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    const long long t = (long long)block * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const int q = (int)(t % NRHS);
     if (!sc[q].active) return;
@@ -1327,7 +1328,9 @@ cudaError_t bfinish_on(gbds_bsolver b, int mode, cudaStream_t st) {
 int packed_variant(gbds_bsolver b) { return b->nrhs >= 16 ? 3 : b->nrhs == 8 ? 2 : 0; }
 
 // out = in - kappa^2 D_eo D_oe in for all rhs (partials: per-rhs |out|^2)
-cudaError_t apply_Mb(gbds_bsolver b, const void *in, void *out, int isign, double *partials, cudaStream_t st) {
+// flip: the direction of the first of the two launches (the second's is the other)
+cudaError_t apply_Mb(gbds_bsolver b, const void *in, void *out, int isign, double *partials, cudaStream_t st,
+                     bool flip = false) {
     gbds_solver s = b->s1;
     const float k2 = (float)(s->prm.kappa * s->prm.kappa);
     // inner fields in FP32 spin pairs: the fully packed FP32x2 kernel from 8
@@ -1335,9 +1338,10 @@ cudaError_t apply_Mb(gbds_bsolver b, const void *in, void *out, int isign, doubl
     // there is no epilogue
     const int v = b->nrhs >= 8 ? 2 : 0;
     cudaError_t e = launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, in, b->t, isign, 0, nullptr, 0.f,
-                                    nullptr, st, packed_variant(b));
+                                    nullptr, st, packed_variant(b), flip);
     if (e != cudaSuccess) return e;
-    return launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, b->t, out, isign, 1, in, -k2, partials, st, v);
+    return launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, b->t, out, isign, 1, in, -k2, partials, st, v,
+                           !flip);
 }
 
 // The fully packed operator (8, 16, 32 rhs) fuses the CG's r -= alpha Ap into
@@ -1345,15 +1349,15 @@ cudaError_t apply_Mb(gbds_bsolver b, const void *in, void *out, int isign, doubl
 bool fused_update(gbds_bsolver b) { return b->nrhs >= 8; }
 
 // r -= alpha_r M^+ in for all active rhs, per-rhs |r|^2 partials
-cudaError_t apply_Mb_dagger_update(gbds_bsolver b, const void *in, cudaStream_t st) {
+cudaError_t apply_Mb_dagger_update(gbds_bsolver b, const void *in, cudaStream_t st, bool flip) {
     gbds_solver s = b->s1;
     const float k2 = (float)(s->prm.kappa * s->prm.kappa);
     cudaError_t e =
         launch_gen_f32p(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, in, b->t, -1, 0, nullptr, 0.f, nullptr, st,
-                        packed_variant(b));
+                        packed_variant(b), flip);
     if (e != cudaSuccess) return e;
     return launch_gen_f32p_cg_update(b->gm, s->prm.inner_recon, b->nrhs, s->gauge32, b->t, -1, 1, in, -k2, b->bsc, b->r,
-                                     b->bpartials, st);
+                                     b->bpartials, st, !flip);
 }
 
 cudaError_t read_bscalars(gbds_bsolver b, cudaStream_t st) {
@@ -1363,17 +1367,18 @@ cudaError_t read_bscalars(gbds_bsolver b, cudaStream_t st) {
 }
 
 // One iteration of the lockstep CG (7 launches, 8 without the fused update).
-cudaError_t bcg_iteration(gbds_bsolver b, cudaStream_t st) {
+// flip alternates: an iteration's five passes over the fields alternate too.
+cudaError_t bcg_iteration(gbds_bsolver b, cudaStream_t st, bool flip) {
     const long long n = bcount(b);
     const int nb = bblocks(b);
     const size_t cs = bcs(b);
     const int nr = b->nrhs;
-    cudaError_t e = apply_Mb(b, b->p, b->Mp, +1, b->bpartials, st);
+    cudaError_t e = apply_Mb(b, b->p, b->Mp, +1, b->bpartials, st, flip);
     if (e == cudaSuccess) e = bfinish_on(b, kBAlpha, st);
     if (e == cudaSuccess && fused_update(b)) {
-        e = apply_Mb_dagger_update(b, b->Mp, st);
+        e = apply_Mb_dagger_update(b, b->Mp, st, flip);
     } else if (e == cudaSuccess) {
-        e = apply_Mb(b, b->Mp, b->Ap, -1, nullptr, st);
+        e = apply_Mb(b, b->Mp, b->Ap, -1, nullptr, st, flip);
         if (e != cudaSuccess) return e;
 #define GBDS_UPD(NR)                                                                                      \
     launch_pdl(bcg_update<NR>, dim3(nb), 128, st, static_cast<float4 *>(b->r), static_cast<const float4 *>(b->Ap), \
@@ -1387,7 +1392,7 @@ cudaError_t bcg_iteration(gbds_bsolver b, cudaStream_t st) {
     if (e != cudaSuccess) return e;
 #define GBDS_XP(NR)                                                                                         \
     launch_pdl(bcg_xpay<NR>, dim3(nb), 128, st, static_cast<float4 *>(b->e), static_cast<const float4 *>(b->r), \
-               static_cast<float4 *>(b->p), (const BScalars *)b->bsc, n, cs)
+               static_cast<float4 *>(b->p), (const BScalars *)b->bsc, n, cs, (int)flip)
     GBDS_BN(nr, GBDS_XP)
 #undef GBDS_XP
     count_launch();
@@ -1412,7 +1417,7 @@ cudaError_t bcg(gbds_bsolver b, const std::vector<double> &target, int max_iter,
             e = launch(b->steps, st);
             done = kCheck;
         } else {
-            e = bcg_iteration(b, st);
+            e = bcg_iteration(b, st, k & 1);
         }
         if (e != cudaSuccess) break;
         k += done;
@@ -1490,7 +1495,7 @@ extern "C" int gbds_bsolver_create(gbds_bsolver *out, const int dims[4], int nrh
     if (e == cudaSuccess)
         record(b->steps, kCheck * (fused_update(b) ? 7 : 8), [&](cudaStream_t cs) {
             cudaError_t le = cudaSuccess;
-            for (int i = 0; i < kCheck && le == cudaSuccess; i++) le = bcg_iteration(b, cs);
+            for (int i = 0; i < kCheck && le == cudaSuccess; i++) le = bcg_iteration(b, cs, i & 1);
             return le;
         });
     if (e != cudaSuccess) {
