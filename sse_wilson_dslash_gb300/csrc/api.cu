@@ -3,6 +3,7 @@
 // (init / free / apply / pack) behind precision-suffixed names.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <cstdio>
@@ -547,6 +548,8 @@ extern "C" int gbds_op_dslash(gbds_op op, const void *gauge, const void *psi, vo
 
 namespace {
 
+constexpr int kLegacyParts = 12;  // of direct calls (direct_parts)
+
 struct LegacyCtx {
     int refcount = 0;
     gbds_op op = nullptr;
@@ -559,6 +562,8 @@ struct LegacyCtx {
     void *d_psi = nullptr;         // internal, one checkerboard
     void *d_res = nullptr;         // internal, one checkerboard
     const void *cached_u = nullptr;
+    cudaStream_t result_stream = nullptr;  // direct calls in parts (direct_apply)
+    cudaEvent_t packed[kLegacyParts] = {};
 };
 
 LegacyCtx g_legacy[2][2];  // [prec 32 -> 0, 64 -> 1][nd 4 -> 0, 3 -> 1]
@@ -573,7 +578,8 @@ int g_last_path = -1;   // 0 staged, 1 direct
 // view; on a coherent host (NVLink-C2C with address translation services) the
 // GPU reads pageable memory through the host page tables; device and managed
 // pointers are usable as they are.
-const void *device_view(const void *p) {
+// *host: it is host memory.
+const void *device_view(const void *p, bool *host = nullptr) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
@@ -582,13 +588,16 @@ const void *device_view(const void *p) {
     switch (a.type) {
     case cudaMemoryTypeDevice:
     case cudaMemoryTypeManaged: return p;
-    case cudaMemoryTypeHost: return a.devicePointer;
+    case cudaMemoryTypeHost:
+        if (host) *host = true;
+        return a.devicePointer;
     default: break;
     }
     int dev = 0, pageable = 0, ats = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev);
     cudaDeviceGetAttribute(&ats, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
+    if (host) *host = true;
     return (pageable && ats) ? p : nullptr;
 }
 
@@ -596,10 +605,14 @@ LegacyCtx &ctx_for(int prec, int nd) { return g_legacy[prec == 32 ? 0 : 1][nd ==
 
 void legacy_release(LegacyCtx &c) {
     if (c.stream) cudaStreamSynchronize(c.stream);
+    if (c.result_stream) cudaStreamSynchronize(c.result_stream);
     void *bufs[] = {c.d_u_packed, c.d_gauge, c.d_psi_packed, c.d_res_packed, c.d_psi, c.d_res};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (c.stream) cudaStreamDestroy(c.stream);
+    if (c.result_stream) cudaStreamDestroy(c.result_stream);
+    for (cudaEvent_t ev : c.packed)
+        if (ev) cudaEventDestroy(ev);
     gbds_op_destroy(c.op);
     c = LegacyCtx();
 }
@@ -676,7 +689,12 @@ void legacy_init(int prec, int nd, const int *latt_size, void (*getSiteCoords)(i
     n.canonical = canonical;
     const size_t real = prec == 32 ? 4 : 8;
     const size_t spin_sites = canonical ? (size_t)g.Vh : (size_t)g.V;
+    int least = 0, greatest = 0;
     cudaError_t e = cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&n.result_stream, cudaStreamNonBlocking, greatest);
+    for (cudaEvent_t &ev : n.packed)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc(&n.d_u_packed, (size_t)g.V * 4 * 18 * real);
     if (e == cudaSuccess) e = cudaMalloc(&n.d_gauge, gbds_op_gauge_bytes(n.op));
     if (e == cudaSuccess) e = cudaMalloc(&n.d_psi_packed, spin_sites * 24 * real);
@@ -698,6 +716,76 @@ void legacy_free(int prec, int nd) {
     LegacyCtx &c = ctx_for(prec, nd);
     if (c.refcount == 0) return;
     if (--c.refcount == 0) legacy_release(c);
+}
+
+cudaError_t legacy_dslash(const LegacyCtx &c, int prec, int isign, int cb, cudaStream_t s, const SiteRange &range = {}) {
+    const gbds_op_s &op = *c.op;
+    return prec == 32 ? launch_dslash_f32(op.g, op.recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, op.block, op.variant, s, range)
+                      : launch_dslash_f64(op.g, op.recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, s, range);
+}
+
+// In how many parts a direct call on host links goes.  The link to the host
+// (211 GB/s either way measured, whatever reads it; 191 MB of links in FP32 at
+// 24^3x48) bounds the call, so the operator and the results of one part of the
+// lattice go while the links of the next come in.  A part costs about 8 us (the
+// operator and the two layout launches run at its size) and leaves 1/parts of
+// the operator and the results without links to hide behind: the best number
+// goes with the square root of the size.  us a call (start: 24^3x48 FP32 1290,
+// FP64 2972; 16^3x32 278, 626):
+//   parts            1      2      3      4      6      8
+//   24^3x48 FP32  1302   1238   1208   1182   1206   1211
+//   24^3x48 FP64  2650   2594   2514   2429   2396   2347
+//   16^3x32 FP32   273    272    276    281    296    310
+//   16^3x32 FP64   544    536    516    521    538    575
+int direct_parts(const Geom &g, int prec) {
+    const size_t link_bytes = (size_t)g.V * g.nd * 18 * (prec == 32 ? 4 : 8);
+    const int most = std::min(kLegacyParts, g.L[g.nd - 1] - 1);
+    int parts = 1;
+    while (parts < most && (size_t)(parts + 1) * (parts + 1) * 8000000 <= link_bytes) parts++;
+    return parts;
+}
+
+// A call on arrays that the kernels reach where they lie.  du == nullptr: the
+// links of the call before are still in place.  Small lattices are bound by
+// launches: spinor and links come in with one, and the others overlap their
+// predecessor's end (8^4 FP32 42 -> 29 us a call).
+cudaError_t direct_apply(LegacyCtx &c, int prec, const void *du, const void *dpsi, void *dres, int isign, int cb,
+                         int parts) {
+    const Geom &g = c.op->g;
+    const int recon = c.op->recon, target = 1 - cb;
+    cudaStream_t s = c.stream, t = c.stream;
+    cudaError_t e = cudaSuccess;
+    auto finish = [&](const SiteRange &range) {
+        if (e == cudaSuccess) e = legacy_dslash(c, prec, isign, cb, t, range);
+        if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, nullptr, 0, target, dres, t, false, range);
+    };
+    if (!du) parts = 1;
+    if (!du) e = launch_pack_spinor(g, prec, dpsi, nullptr, 0, cb, c.d_psi, s);
+    else if (parts <= 1) e = launch_pack_fields(g, prec, recon, du, c.d_gauge, {}, dpsi, cb, c.d_psi, s);
+    if (parts <= 1) {
+        finish({});
+    } else {
+        // slices of the slowest lattice direction are contiguous sites
+        t = c.result_stream;
+        const int slices = g.L[g.nd - 1], per = g.Vh / slices;
+        e = launch_pack_fields(g, prec, recon, du, c.d_gauge, {(slices - 1) * per, per}, dpsi, cb, c.d_psi, s);
+        for (int p = 0; p < parts && e == cudaSuccess; p++) {
+            const int s0 = (int)((long long)slices * p / parts), s1 = (int)((long long)slices * (p + 1) / parts);
+            const int n = std::min(s1, slices - 1) - s0;
+            if (n > 0) e = launch_pack_fields(g, prec, recon, du, c.d_gauge, {s0 * per, n * per}, nullptr, cb, nullptr, s, true);
+            if (e == cudaSuccess) e = cudaEventRecord(c.packed[p], s);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(t, c.packed[p], 0);
+            finish({s0 * per, (s1 - s0) * per});
+        }
+    }
+    // result_stream waits for the other through the events
+    const cudaError_t e2 = cudaStreamSynchronize(t);
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(s);
+    } else {
+        e = e2;
+    }
+    return e;
 }
 
 void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, int isign, int cb, const char *fn) {
@@ -724,9 +812,10 @@ void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, i
     cudaError_t e = cudaSuccess;
     const bool reuse_gauge = g_gauge_cache && c.cached_u == u;
     const void *du = nullptr, *dpsi = nullptr;
+    bool host_links = false;
     void *dres = nullptr;
     if (c.canonical && g_host_access == 0) {
-        du = reuse_gauge ? u : device_view(u);
+        du = reuse_gauge ? u : device_view(u, &host_links);
         dpsi = device_view(psi);
         dres = const_cast<void *>(device_view(res));
     }
@@ -735,17 +824,12 @@ void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, i
     if (du && dpsi && dres && aligned) {
         // Direct: the layout kernels read u and psi and write res where they
         // lie, with no intermediate copy.
-        if (!reuse_gauge) {
-            e = launch_pack_gauge(g, prec, c.op->recon, du, nullptr, c.d_gauge, s);
-            c.cached_u = e == cudaSuccess ? u : nullptr;
-        }
-        if (e == cudaSuccess) e = launch_pack_spinor(g, prec, dpsi, nullptr, 0, cb, c.d_psi, s);
-        if (e == cudaSuccess)
-            e = prec == 32 ? launch_dslash_f32(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s)
-                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, s);
-        if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, nullptr, 0, target, dres, s);
-        cudaError_t e2 = cudaStreamSynchronize(s);
-        if (e == cudaSuccess) e = e2;
+        // Not in parts where results would overwrite links still to be read.
+        const uintptr_t ub = reinterpret_cast<uintptr_t>(du), rb = reinterpret_cast<uintptr_t>(dres);
+        const bool apart = ub + (size_t)g.V * 72 * real <= rb || rb + (size_t)g.V * spinor <= ub;
+        const int parts = host_links && apart ? direct_parts(g, prec) : 1;
+        e = direct_apply(c, prec, reuse_gauge ? nullptr : du, dpsi, dres, isign, cb, parts);
+        if (!reuse_gauge) c.cached_u = e == cudaSuccess ? u : nullptr;
         g_last_path = 1;
         if (e != cudaSuccess) {
             c.cached_u = nullptr;
@@ -764,9 +848,7 @@ void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, i
         const char *src = static_cast<const char *>(psi) + (size_t)cb * g.Vh * spinor;
         if (e == cudaSuccess) e = cudaMemcpyAsync(c.d_psi_packed, src, (size_t)g.Vh * spinor, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = launch_pack_spinor(g, prec, c.d_psi_packed, nullptr, cb * g.Vh, cb, c.d_psi, s);
-        if (e == cudaSuccess)
-            e = prec == 32 ? launch_dslash_f32(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s)
-                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, s);
+        if (e == cudaSuccess) e = legacy_dslash(c, prec, isign, cb, s);
         if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, nullptr, target * g.Vh, target, c.d_res_packed, s);
         char *dst = static_cast<char *>(res) + (size_t)target * g.Vh * spinor;
         if (e == cudaSuccess) e = cudaMemcpyAsync(dst, c.d_res_packed, (size_t)g.Vh * spinor, cudaMemcpyDeviceToHost, s);
@@ -776,9 +858,7 @@ void legacy_apply(int prec, int nd, const void *u, const void *psi, void *res, i
         if (e == cudaSuccess) e = cudaMemcpyAsync(c.d_psi_packed, psi, (size_t)g.V * spinor, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(c.d_res_packed, res, (size_t)g.V * spinor, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = launch_pack_spinor(g, prec, c.d_psi_packed, table, 0, cb, c.d_psi, s);
-        if (e == cudaSuccess)
-            e = prec == 32 ? launch_dslash_f32(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, c.op->block, c.op->variant, s)
-                           : launch_dslash_f64(g, c.op->recon, c.d_gauge, c.d_psi, c.d_res, isign, cb, s);
+        if (e == cudaSuccess) e = legacy_dslash(c, prec, isign, cb, s);
         if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, table, 0, target, c.d_res_packed, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(res, c.d_res_packed, (size_t)g.V * spinor, cudaMemcpyDeviceToHost, s);
     }

@@ -14,7 +14,8 @@ cudaError_t launch_split(const DslashArgs<float> &a, int isign, cudaStream_t st,
     return cudaGetLastError();
 }
 
-DslashArgs<float> f32_args(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int cb) {
+DslashArgs<float> f32_args(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int cb,
+                           const SiteRange &range = {}) {
     DslashArgs<float> a;
     a.g = g;
     a.psi = static_cast<const float4 *>(psi);
@@ -22,7 +23,19 @@ DslashArgs<float> f32_args(const Geom &g, int recon, const void *gauge, const vo
     a.gauge = static_cast<const char *>(gauge);
     a.link_block_bytes = (size_t)recon * 4 * g.stride;
     a.pt = 1 - cb;
+    a.first = range.first;
+    a.end = range.end(g);
     return a;
+}
+
+// Part of a lattice, registers capped for 6 CTAs per SM.
+template <int ND, int RECON>
+cudaError_t launch_range(const DslashArgs<float> &a, int isign, cudaStream_t st) {
+    const dim3 grid((a.end - a.first + 127) / 128);
+    if (isign > 0) launch_pdl(dslash_kernel<float, ND, RECON, 1, 6, true>, grid, 128, st, a);
+    else launch_pdl(dslash_kernel<float, ND, RECON, -1, 6, true>, grid, 128, st, a);
+    count_launch();
+    return cudaGetLastError();
 }
 
 // Four warps a site: the variant after the register caps.
@@ -63,7 +76,12 @@ void f32_tuning(const Geom &g, int recon, int *block, int *variant) {
 }
 
 cudaError_t launch_dslash_f32(const Geom &g, int recon, const void *gauge, const void *psi, void *res,
-                              int isign, int cb, int block, int variant, cudaStream_t stream) {
+                              int isign, int cb, int block, int variant, cudaStream_t stream, const SiteRange &range) {
+    if (range.count >= 0) {
+        const DslashArgs<float> a = f32_args(g, recon, gauge, psi, res, cb, range);
+        if (g.nd == 4) return recon == 18 ? launch_range<4, 18>(a, isign, stream) : launch_range<4, 12>(a, isign, stream);
+        return recon == 18 ? launch_range<3, 18>(a, isign, stream) : launch_range<3, 12>(a, isign, stream);
+    }
     if (variant == kSplitVariant) {
         const DslashArgs<float> a = f32_args(g, recon, gauge, psi, res, cb);
         if (g.nd == 4) return recon == 18 ? launch_split<4, 18>(a, isign, stream) : launch_split<4, 12>(a, isign, stream);

@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(96 * GROUPS, GROUPS == 1 ? 7 : 2)
     th.lane = threadIdx.x & 31;
     th.grp = GROUPS == 1 ? 0 : warp / 3;
     th.c = GROUPS == 1 ? warp : warp % 3;
-    const int h = (blockIdx.x * GROUPS + th.grp) * kFxSites + th.lane;
-    th.act = h < a.g.Vh;
+    const int h = a.first + (blockIdx.x * GROUPS + th.grp) * kFxSites + th.lane;
+    th.act = h < a.end;
     Nbr n;
     if (th.act) neighbours<ND>(a.g, h, a.pt, n);
     th.pol = l2_evict_first_policy();
@@ -340,7 +340,8 @@ __global__ void __launch_bounds__(96 * GROUPS, GROUPS == 1 ? 7 : 2)
     }
 }
 
-DslashArgs<double> f64_args(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int cb) {
+DslashArgs<double> f64_args(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int cb,
+                            const SiteRange &range = {}) {
     DslashArgs<double> a;
     a.g = g;
     a.psi = static_cast<const double2 *>(psi);
@@ -348,13 +349,15 @@ DslashArgs<double> f64_args(const Geom &g, int recon, const void *gauge, const v
     a.gauge = static_cast<const char *>(gauge);
     a.link_block_bytes = (size_t)Field<double>::link_vecs(recon) * g.stride * 16;
     a.pt = 1 - cb;
+    a.first = range.first;
+    a.end = range.end(g);
     return a;
 }
 
 template <int ND, int RECON, int EPI, int GROUPS>
 cudaError_t launch_fx(const DslashArgs<double> &a, int isign, const double2 *x, double coef, double *partials,
                       cudaStream_t st, const CgUpdate<double> &upd = {}) {
-    const dim3 grid((a.g.Vh + kFxSites * GROUPS - 1) / (kFxSites * GROUPS));
+    const dim3 grid((a.end - a.first + kFxSites * GROUPS - 1) / (kFxSites * GROUPS));
     const int threads = 96 * GROUPS;
     if (isign > 0) launch_pdl(dslash_fx_kernel<ND, RECON, 1, EPI, GROUPS>, grid, threads, st, a, x, coef, upd, partials);
     else launch_pdl(dslash_fx_kernel<ND, RECON, -1, EPI, GROUPS>, grid, threads, st, a, x, coef, upd, partials);
@@ -367,8 +370,8 @@ cudaError_t launch_fx(const DslashArgs<double> &a, int isign, const double2 *x, 
 // FP64 has one kernel and launch shape: block and variant are accepted and
 // make no difference.
 cudaError_t launch_dslash_f64(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign, int cb,
-                              cudaStream_t stream) {
-    const DslashArgs<double> a = f64_args(g, recon, gauge, psi, res, cb);
+                              cudaStream_t stream, const SiteRange &range) {
+    const DslashArgs<double> a = f64_args(g, recon, gauge, psi, res, cb, range);
     if (g.nd == 4)
         return recon == 18 ? launch_fx<4, 18, 0, 1>(a, isign, nullptr, 0.0, nullptr, stream)
                            : launch_fx<4, 12, 0, 1>(a, isign, nullptr, 0.0, nullptr, stream);

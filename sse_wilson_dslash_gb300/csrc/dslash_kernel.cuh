@@ -17,6 +17,7 @@
 
 #include "dfloat.cuh"
 #include "gbds_internal.h"
+#include "pdl.cuh"
 
 namespace gbds {
 
@@ -372,6 +373,7 @@ struct DslashArgs {
     const char *gauge;                // both checkerboards
     size_t link_block_bytes;          // bytes of one (parity, mu) block
     int pt;                           // target parity = 1 - cb
+    int first, end;                   // target sites (where a launch takes a SiteRange)
 };
 
 template <typename T, int ND, int RECON, int ISIGN, int MU>
@@ -442,22 +444,18 @@ __device__ __forceinline__ void hop_pair_any(const DslashArgs<T> &a, int h, cons
 template <int MINB> struct Bounds { static constexpr int threads = 128, blocks = MINB; };
 template <> struct Bounds<0> { static constexpr int threads = 256, blocks = 1; };
 
-// Programmatic dependent launch: the next kernel launched on the stream with
-// the programmatic-serialisation attribute may start its blocks once every
-// block of this grid has started; it waits (griddepcontrol.wait) for this
-// grid's completion and memory before its first global read.  Without the
-// attribute both instructions are no-ops.
-__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait_prev() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <typename T, int ND, int RECON, int ISIGN, int MINB>
+// RANGE: sites [a.first, a.end) only (an instance of its own: the offset costs
+// the whole-lattice one 1.5 % at 32^3x64).
+template <typename T, int ND, int RECON, int ISIGN, int MINB, bool RANGE = false>
 __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks) dslash_kernel(const DslashArgs<T> a) {
     pdl_allow_next();
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    int h = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (RANGE) h += a.first;
+    const int end = RANGE ? a.end : a.g.Vh;
     Nbr n;
-    if (h < a.g.Vh) neighbours<ND>(a.g, h, a.pt, n);  // index arithmetic only: overlaps the previous grid
+    if (h < end) neighbours<ND>(a.g, h, a.pt, n);  // index arithmetic only: overlaps the previous grid
     pdl_wait_prev();
-    if (h >= a.g.Vh) return;
+    if (h >= end) return;
     cx<T> acc[4][3];
 #pragma unroll
     for (int s = 0; s < 4; s++)
@@ -476,29 +474,6 @@ template <> struct Variants<float> { static constexpr int n = 5; static constexp
 // double-float at 32^3x64: 1.28 ms uncapped, 0.86 ms at 3 and 0.74 ms at 4
 // CTAs of 128 threads per SM; 5 and 6 spill 1.2-1.9 KB and lose
 template <> struct Variants<dfloat> { static constexpr int n = 3; static constexpr int minb[3] = {0, 3, 4}; };
-
-// Launch with the programmatic-serialisation attribute (see pdl_wait_prev).
-template <typename... P, typename... A>
-void launch_pdl_smem(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, const A &...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    // a failed launch also sets the runtime's last error, which every
-    // launcher returns through cudaGetLastError()
-    (void)cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
-template <typename... P, typename... A>
-void launch_pdl(void (*kernel)(P...), dim3 grid, int block, cudaStream_t stream, const A &...args) {
-    launch_pdl_smem(kernel, grid, block, 0, stream, args...);
-}
 
 template <typename T, int MINB>
 void launch_variant(const DslashArgs<T> &a, dim3 grid, int block, int nd, int recon, int isign, cudaStream_t stream) {

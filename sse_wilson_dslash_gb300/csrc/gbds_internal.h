@@ -32,6 +32,12 @@ int set_error(int code, const std::string &msg);
 int cuda_error(cudaError_t e, const char *where);
 void count_launch(int n = 1);
 
+// Target sites [first, first + count) of a launch; count < 0: to the last one.
+struct SiteRange {
+    int first = 0, count = -1;
+    int end(const Geom &g) const { return count < 0 ? g.Vh : first + count; }
+};
+
 // Launchers (defined in dslash_f32.cu / dslash_f64.cu / layout.cu).
 // All pointers are device pointers; `stream` is a cudaStream_t.
 // block: threads per block (0 = default); variant: register-cap variant
@@ -39,10 +45,11 @@ void count_launch(int n = 1);
 // site.  f32_tuning: the ones for a lattice.
 void f32_tuning(const Geom &g, int recon, int *block, int *variant);
 cudaError_t launch_dslash_f32(const Geom &g, int recon, const void *gauge, const void *psi,
-                              void *res, int isign, int cb, int block, int variant, cudaStream_t stream);
+                              void *res, int isign, int cb, int block, int variant, cudaStream_t stream,
+                              const SiteRange &range = {});
 // FP64: one kernel and launch shape (dslash_f64.cu)
 cudaError_t launch_dslash_f64(const Geom &g, int recon, const void *gauge, const void *psi,
-                              void *res, int isign, int cb, cudaStream_t stream);
+                              void *res, int isign, int cb, cudaStream_t stream, const SiteRange &range = {});
 // variant indices the tuning calls accept (FP64: three, all the same kernel)
 int dslash_variants(int prec);
 
@@ -100,9 +107,17 @@ cudaError_t launch_f64_to_df(const void *in, void *out, size_t n, cudaStream_t s
 cudaError_t launch_pack_spinor(const Geom &g, int prec, const void *psi_packed, const int *site_table,
                                int site0, int parity, void *spinor, cudaStream_t stream, bool df = false);
 cudaError_t launch_unpack_spinor(const Geom &g, int prec, const void *spinor, const int *site_table,
-                                 int site0, int parity, void *psi_packed, cudaStream_t stream, bool df = false);
+                                 int site0, int parity, void *psi_packed, cudaStream_t stream, bool df = false,
+                                 const SiteRange &range = {});
 cudaError_t launch_pack_gauge(const Geom &g, int prec, int recon, const void *u_packed,
                               const int *site_table, void *gauge, cudaStream_t stream);
+// Canonical order, in one launch: the links of the sites `range` of both
+// checkerboards and, if psi_packed (a full lattice) is not null, checkerboard
+// `parity` of the spinor.  chained: after another of these on the stream, of
+// other sites, whose last blocks it may overlap.
+cudaError_t launch_pack_fields(const Geom &g, int prec, int recon, const void *u_packed, void *gauge,
+                               const SiteRange &range, const void *psi_packed, int parity, void *spinor,
+                               cudaStream_t stream, bool chained = false);
 
 // Generalised Dslash (dslash_gen_*.cu): FP32 arithmetic and links, nrhs in
 // {1,2,4,8,16,32}, spinor formats 0 FP32, 1 BF16, 2 FP16 + norm, 3 FP32 in

@@ -13,6 +13,7 @@
 
 #include "dfloat.cuh"
 #include "gbds_internal.h"
+#include "pdl.cuh"
 
 namespace gbds {
 
@@ -123,12 +124,10 @@ inline unsigned blocks_for(long long n, int threads) { return (unsigned)((n + th
 constexpr int kSpinorTile = 128;  // sites per block
 constexpr int kGaugeTile = 32;
 
-// packed: first site of checkerboard `parity` (sites [0, Vh) of that half).
-template <int UNITS, bool DF = false>
-__global__ void __launch_bounds__(128) pack_spinor_tile(const uint4 *packed, int Vh, int stride, uint4 *__restrict__ soa) {
-    __shared__ uint4 sm[kSpinorTile * UNITS];
-    const int h0 = blockIdx.x * kSpinorTile;
-    const int n = min(kSpinorTile, Vh - h0);
+// Sites [h0, h0 + n) of a checkerboard, of which `packed` is the first site.
+template <int UNITS, bool DF>
+__device__ __forceinline__ void pack_spinor_block(const uint4 *packed, int h0, int n, int stride, uint4 *__restrict__ soa,
+                                                  uint4 *sm) {
     const uint4 *src = packed + (size_t)h0 * UNITS;
     for (int e = threadIdx.x; e < n * UNITS; e += blockDim.x) sm[e] = src[e];
     __syncthreads();
@@ -139,10 +138,20 @@ __global__ void __launch_bounds__(128) pack_spinor_tile(const uint4 *packed, int
 }
 
 template <int UNITS, bool DF = false>
-__global__ void __launch_bounds__(128) unpack_spinor_tile(const uint4 *__restrict__ soa, int Vh, int stride, uint4 *packed) {
+__global__ void __launch_bounds__(128) pack_spinor_tile(const uint4 *packed, int Vh, int stride, uint4 *__restrict__ soa) {
     __shared__ uint4 sm[kSpinorTile * UNITS];
     const int h0 = blockIdx.x * kSpinorTile;
-    const int n = min(kSpinorTile, Vh - h0);
+    pack_spinor_block<UNITS, DF>(packed, h0, min(kSpinorTile, Vh - h0), stride, soa, sm);
+}
+
+// sites [first, end)
+template <int UNITS, bool DF = false>
+__global__ void __launch_bounds__(128) unpack_spinor_tile(const uint4 *__restrict__ soa, int first, int end, int stride,
+                                                          uint4 *packed) {
+    __shared__ uint4 sm[kSpinorTile * UNITS];
+    const int h0 = first + blockIdx.x * kSpinorTile;
+    const int n = min(kSpinorTile, end - h0);
+    pdl_wait_prev();
     for (int e = threadIdx.x; e < n * UNITS; e += blockDim.x) {
         const int k = e / n, t = e - k * n;
         sm[t * UNITS + k] = to_packed<DF>(__ldg(soa + (size_t)k * stride + h0 + t));
@@ -152,31 +161,28 @@ __global__ void __launch_bounds__(128) unpack_spinor_tile(const uint4 *__restric
     for (int e = threadIdx.x; e < n * UNITS; e += blockDim.x) dst[e] = sm[e];
 }
 
-// Gauge: block of kGaugeTile consecutive caller sites (canonical order, both
-// checkerboards), only the first nd links of each site are read.  Units of 8
+// Gauge: block of kGaugeTile consecutive caller sites (canonical order, one
+// checkerboard), only the first nd links of each site are read.  Units of 8
 // bytes (one float2 / one double) keep the 3D skip of mu = 3 exact.
 template <typename T, int RECON>
-__global__ void __launch_bounds__(128) pack_gauge_tile(const unsigned long long *packed, Geom g, char *__restrict__ gauge,
-                                                        size_t block_bytes) {
+__device__ __forceinline__ void pack_gauge_block(const unsigned long long *packed, const Geom &g, int p, int h0, int n,
+                                                 char *__restrict__ gauge, size_t block_bytes, unsigned long long *sm) {
     constexpr int SITE_UNITS = 4 * 18 * sizeof(T) / 8;  // 8-byte units per site (4 links)
     constexpr int LINK_UNITS = 18 * sizeof(T) / 8;
-    __shared__ unsigned long long sm[kGaugeTile * SITE_UNITS];
-    const int i0 = blockIdx.x * kGaugeTile;
-    const int n = min(kGaugeTile, g.V - i0);
     const int used = g.nd * LINK_UNITS;  // leading units of each site that are read
-    const unsigned long long *src = packed + (size_t)i0 * SITE_UNITS;
+    const unsigned long long *src = packed + ((size_t)p * g.Vh + h0) * SITE_UNITS;
     for (int e = threadIdx.x; e < n * used; e += blockDim.x) {
         const int t = e / used, u = e - t * used;
         sm[t * SITE_UNITS + u] = src[(size_t)t * SITE_UNITS + u];
     }
+    pdl_wait_prev();  // so that this grid ends after the one before
     __syncthreads();
     const T *st = reinterpret_cast<const T *>(sm);
     constexpr int C = sizeof(T) == 4 ? (RECON == 18 ? 9 : 3) : (RECON == 18 ? 9 : 6);
     for (int e = threadIdx.x; e < n * g.nd * C; e += blockDim.x) {
         const int t = e % n, rest = e / n;
         const int mu = rest / C, k = rest % C;
-        const int i = i0 + t;
-        const int p = i >= g.Vh ? 1 : 0, h = i - p * g.Vh;
+        const int h = h0 + t;
         const T *m = st + (size_t)t * 72 + mu * 18;  // m[(3j+i)*2] = U_ij
         char *blk = gauge + (size_t)(p * g.nd + mu) * block_bytes;
         if constexpr (sizeof(T) == 4 && RECON == 18) {
@@ -192,6 +198,40 @@ __global__ void __launch_bounds__(128) pack_gauge_tile(const unsigned long long 
             reinterpret_cast<double2 *>(blk)[(size_t)k * g.stride + h] = make_double2(m[(3 * c + r) * 2], m[(3 * c + r) * 2 + 1]);
         }
     }
+}
+
+// The first spinor_blocks blocks move a spinor, the others the links of sites
+// [first, end) of both checkerboards, ceil((end - first) / kGaugeTile) blocks each.
+template <typename T, int RECON>
+__global__ void __launch_bounds__(128) pack_fields_tile(const uint4 *psi, uint4 *__restrict__ soa, int spinor_blocks,
+                                                         const unsigned long long *links, const Geom g,
+                                                         char *__restrict__ gauge, size_t block_bytes, int first, int end) {
+    extern __shared__ uint4 tile[];
+    pdl_allow_next();
+    int b = blockIdx.x;
+    if (b < spinor_blocks) {
+        const int h0 = b * kSpinorTile;
+        pack_spinor_block<24 * sizeof(T) / 16, false>(psi, h0, min(kSpinorTile, g.Vh - h0), g.stride, soa, tile);
+        return;
+    }
+    b -= spinor_blocks;
+    const int per = (end - first + kGaugeTile - 1) / kGaugeTile;
+    const int p = b >= per ? 1 : 0;
+    const int h0 = first + (b - p * per) * kGaugeTile;
+    pack_gauge_block<T, RECON>(links, g, p, h0, min(kGaugeTile, end - h0), gauge, block_bytes,
+                               reinterpret_cast<unsigned long long *>(tile));
+}
+
+template <typename T, int RECON>
+void launch_pack_tile(const Geom &g, const uint4 *psi, uint4 *soa, const unsigned long long *links, char *gauge,
+                      size_t block_bytes, int first, int end, cudaStream_t st, bool chained) {
+    const int ns = psi ? (int)blocks_for(g.Vh, kSpinorTile) : 0;
+    const unsigned nl = 2 * blocks_for(end - first, kGaugeTile);
+    const size_t smem = (size_t)sizeof(T) * (ns ? kSpinorTile * 24 : kGaugeTile * 72);
+    if (chained)
+        launch_pdl_smem(pack_fields_tile<T, RECON>, dim3(ns + nl), 128, smem, st, psi, soa, ns, links, g, gauge, block_bytes, first, end);
+    else
+        pack_fields_tile<T, RECON><<<ns + nl, 128, smem, st>>>(psi, soa, ns, links, g, gauge, block_bytes, first, end);
 }
 
 }  // namespace
@@ -228,16 +268,18 @@ cudaError_t launch_pack_spinor(const Geom &g, int prec, const void *psi_packed, 
 }
 
 cudaError_t launch_unpack_spinor(const Geom &g, int prec, const void *spinor, const int *site_table,
-                                 int site0, int parity, void *psi_packed, cudaStream_t stream, bool df) {
+                                 int site0, int parity, void *psi_packed, cudaStream_t stream, bool df,
+                                 const SiteRange &range) {
     const int units = prec == 32 ? 6 : 12;
     df = df && prec == 64;
     const uint4 *src = static_cast<const uint4 *>(spinor);
     if (!site_table) {
         uint4 *dst = static_cast<uint4 *>(psi_packed) + (size_t)(parity * g.Vh - site0) * units;
-        const unsigned nb = blocks_for(g.Vh, kSpinorTile);
-        if (prec == 32) unpack_spinor_tile<6><<<nb, 128, 0, stream>>>(src, g.Vh, g.stride, dst);
-        else if (df) unpack_spinor_tile<12, true><<<nb, 128, 0, stream>>>(src, g.Vh, g.stride, dst);
-        else unpack_spinor_tile<12><<<nb, 128, 0, stream>>>(src, g.Vh, g.stride, dst);
+        const int first = range.first, end = range.end(g);
+        const dim3 nb(blocks_for(end - first, kSpinorTile));
+        if (prec == 32) launch_pdl(unpack_spinor_tile<6>, nb, 128, stream, src, first, end, g.stride, dst);
+        else if (df) launch_pdl(unpack_spinor_tile<12, true>, nb, 128, stream, src, first, end, g.stride, dst);
+        else launch_pdl(unpack_spinor_tile<12>, nb, 128, stream, src, first, end, g.stride, dst);
         count_launch();
         return cudaGetLastError();
     }
@@ -249,24 +291,33 @@ cudaError_t launch_unpack_spinor(const Geom &g, int prec, const void *spinor, co
     return cudaGetLastError();
 }
 
+cudaError_t launch_pack_fields(const Geom &g, int prec, int recon, const void *u_packed, void *gauge,
+                               const SiteRange &range, const void *psi_packed, int parity, void *spinor,
+                               cudaStream_t stream, bool chained) {
+    const uint4 *psi = static_cast<const uint4 *>(psi_packed);
+    if (psi) psi += (size_t)parity * g.Vh * (prec == 32 ? 6 : 12);
+    uint4 *soa = static_cast<uint4 *>(spinor);
+    const auto *src = static_cast<const unsigned long long *>(u_packed);
+    char *dst = static_cast<char *>(gauge);
+    const size_t bb = gauge_block_bytes(g, prec, recon);
+    const int first = range.first, end = range.end(g);
+    if (prec == 32) {
+        if (recon == 18) launch_pack_tile<float, 18>(g, psi, soa, src, dst, bb, first, end, stream, chained);
+        else launch_pack_tile<float, 12>(g, psi, soa, src, dst, bb, first, end, stream, chained);
+    } else {
+        if (recon == 18) launch_pack_tile<double, 18>(g, psi, soa, src, dst, bb, first, end, stream, chained);
+        else launch_pack_tile<double, 12>(g, psi, soa, src, dst, bb, first, end, stream, chained);
+    }
+    count_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_pack_gauge(const Geom &g, int prec, int recon, const void *u_packed, const int *site_table,
                               void *gauge, cudaStream_t stream) {
     const long long n = 2LL * g.nd * g.Vh;
     const size_t bb = gauge_block_bytes(g, prec, recon);
     char *dst = static_cast<char *>(gauge);
-    if (!site_table) {
-        const unsigned long long *src = static_cast<const unsigned long long *>(u_packed);
-        const unsigned nt = blocks_for(g.V, kGaugeTile);
-        if (prec == 32) {
-            if (recon == 18) pack_gauge_tile<float, 18><<<nt, 128, 0, stream>>>(src, g, dst, bb);
-            else pack_gauge_tile<float, 12><<<nt, 128, 0, stream>>>(src, g, dst, bb);
-        } else {
-            if (recon == 18) pack_gauge_tile<double, 18><<<nt, 128, 0, stream>>>(src, g, dst, bb);
-            else pack_gauge_tile<double, 12><<<nt, 128, 0, stream>>>(src, g, dst, bb);
-        }
-        count_launch();
-        return cudaGetLastError();
-    }
+    if (!site_table) return launch_pack_fields(g, prec, recon, u_packed, gauge, {}, nullptr, 0, nullptr, stream);
     const unsigned nb = blocks_for(n, 128);
     if (prec == 32) {
         const float *src = static_cast<const float *>(u_packed);
