@@ -132,11 +132,16 @@ extern "C" int gbds_op_create(gbds_op *op, const int dims[4], int nd, int prec, 
 // 151 with the plain kernel, 147 packed, half + norm 5: 144 / 121).  With 8 rhs
 // the default stays the plain kernel (half + norm: variant 2); gbds_op_autotune
 // or gbds_op_set_tuning reach the packed ones (FP32 193 / 166, bfloat16 172 / 133).
-static int gen_variant(int nrhs, int format) {
+// FP32 fields of few blocks (plain kernel: 128 pairs of a site and a rhs each)
+// take the plain kernel, whose blocks are shorter: 12 rhs on 12^2x16x24 (2592)
+// 20.8 / 23.9, on 16^3x20 (3840) 39.4 / 36.9; 10 rhs on 16^3x20 (3200) 30.9 /
+// 32.4, on 16^3x32 (5120) 50.8 / 49.6; 24 rhs on 10x14x12x20 (3150) 26.1 / 27.0, on
+// 12^2x16x24 (5184) 48.6 / 44.7.
+static int gen_variant(int nrhs, int format, int Vh) {
     const bool bf16 = format == GBDS_SPINOR_BF16, half = bf16 || format == GBDS_SPINOR_F16_NORM;
     if (nrhs == 16 || nrhs == 32) return half ? 4 : 3;
     if (nrhs == 8) return format == GBDS_SPINOR_F16_NORM ? 2 : 0;
-    if (!half) return nrhs >= 8 ? 2 : 0;
+    if (!half) return nrhs >= 8 && (long long)Vh * nrhs > 3500 * 128 ? 2 : 0;
     if (nrhs % 2 == 0 && nrhs >= 6) return 3;
     return nrhs >= (bf16 ? 9 : 4) ? 2 : 0;
 }
@@ -172,7 +177,7 @@ extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int pre
     // autotune chooses per shape.
     const bool gen = nrhs > 1 || (format != GBDS_SPINOR_NATIVE && format != GBDS_SPINOR_DOUBLE_FLOAT);
     o->block = 128;
-    o->variant = gen ? gen_variant(nrhs, format) : 0;
+    o->variant = gen ? gen_variant(nrhs, format, g.Vh) : 0;
     if (!gen && prec == 32) f32_tuning(g, recon, &o->block, &o->variant);
     if (gen) o->g.zblock = gen_zblock(g, nrhs, format, recon);
     o->tensor_cores = 0;
@@ -757,7 +762,7 @@ cudaError_t direct_apply(LegacyCtx &c, int prec, const void *du, const void *dps
     cudaError_t e = cudaSuccess;
     auto finish = [&](const SiteRange &range) {
         if (e == cudaSuccess) e = legacy_dslash(c, prec, isign, cb, t, range);
-        if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, nullptr, 0, target, dres, t, false, range);
+        if (e == cudaSuccess) e = launch_unpack_spinor(g, prec, c.d_res, nullptr, 0, target, dres, t, false, range, true);
     };
     if (!du) parts = 1;
     if (!du) e = launch_pack_spinor(g, prec, dpsi, nullptr, 0, cb, c.d_psi, s);

@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(96 * GROUPS, GROUPS == 1 ? 7 : 2)
     dslash_fx_kernel(const DslashArgs<double> a, const double2 *__restrict__ x, double coef, const CgUpdate<double> upd,
                      double *partials) {
     __shared__ FxShared<GROUPS> sm;
-    pdl_allow_next();
+    if (gridDim.x > 152 * (GROUPS == 1 ? 7 : 2)) pdl_allow_next();
     const int warp = threadIdx.x >> 5;
     FxThread th;
     th.lane = threadIdx.x & 31;

@@ -388,7 +388,6 @@ __device__ __forceinline__ void su3_mul_splat(const float4 *M, const cx<float> (
 template <int FMT, int RECON, int ISIGN, int NRHS, int EPI>
 __global__ void __launch_bounds__(128, 6) dslash_gen2_kernel(const GenArgs a) {
     static_assert(NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides");
-    pdl_allow_next();
     pdl_wait_prev();
     constexpr int P = 128 / NRHS;  // sites per CTA
     __shared__ float4 sL[P][8][9];
@@ -654,7 +653,6 @@ __device__ __forceinline__ float2 (*staged_links())[8][9] {
 template <int FMT, int RECON, int ISIGN, int NRHS, int EPI>
 __global__ void __launch_bounds__(128, FMT == kFmtF16N && NRHS ? 5 : 7) dslash_gen3_kernel(const GenArgs a) {
     static_assert(NRHS == 0 ? EPI == 0 : NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides, or any count");
-    pdl_allow_next();
     pdl_wait_prev();
     const int nr = nrhs_of<NRHS>(a);
     const int P = 128 / nr;  // sites per CTA
@@ -844,7 +842,6 @@ __device__ __forceinline__ void packed_mul_recon2(const SPLAT *M, const float2 (
 template <int FMT, int RECON, int ISIGN, int NRHS>
 __global__ void __launch_bounds__(128, 4) dslash_gen4_kernel(const GenArgs a) {
     static_assert(NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides");
-    pdl_allow_next();
     pdl_wait_prev();
     constexpr int H = NRHS / 2;    // threads per site
     constexpr int P = 128 / H;     // sites per CTA
@@ -958,7 +955,6 @@ __device__ __forceinline__ void load_reals2(const char *base, size_t cs, size_t 
 
 template <int FMT, int RECON, int ISIGN>
 __global__ void __launch_bounds__(128, 4) dslash_gen4w_kernel(const GenArgs a) {
-    pdl_allow_next();
     pdl_wait_prev();
     const int nr = a.nrhs, H = nr / 2, P = 128 / H;  // threads per site, sites per CTA
     constexpr bool SCALE = FMT == kFmtF16N;
@@ -1096,7 +1092,6 @@ template <int FMT, int RECON, int ISIGN, int NRHS>
 __global__ void __launch_bounds__(128, G5Smem<FMT, NRHS>::MINB) dslash_gen5_kernel(const GenArgs a) {
     static_assert(FMT == kFmtBF16 || FMT == kFmtF16N, "16-bit storage");
     static_assert(NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides");
-    pdl_allow_next();
     pdl_wait_prev();
     using SM = G5Smem<FMT, NRHS>;
     constexpr int H = NRHS / 2;
@@ -1185,7 +1180,6 @@ __global__ void __launch_bounds__(128, G5Smem<FMT, NRHS>::MINB) dslash_gen5_kern
 // rvec instead of the store, with |r|^2.
 template <int FMT, int RECON, int ISIGN, int NRHS, int EPI, int LFMT = 0>
 __global__ void __launch_bounds__(128, 6) dslash_gen_kernel(const GenArgs a) {
-    pdl_allow_next();
     pdl_wait_prev();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int nr = nrhs_of<NRHS>(a);

@@ -599,7 +599,7 @@ template <typename T, int RECON, int ISIGN, int MINB, bool UPD>
 __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks)
     dslash_xpay_kernel(const DslashArgs<T> a, const typename VecOf<T>::S *__restrict__ x, T coef, const CgUpdate<T> upd,
                        double *partials, const SumHere here) {
-    pdl_allow_next();
+    if (MINB || gridDim.x > 2 * 152) pdl_allow_next();
     pdl_wait_prev();
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     T nrm = T(0);
@@ -684,7 +684,6 @@ __global__ void __launch_bounds__(128, 6)
     dslash_split_kernel(const DslashArgs<float> a, const float4 *__restrict__ x, float coef, const CgUpdate<float> upd,
                         double *partials, const SumHere here) {
     __shared__ float4 sm[4][6][32];
-    pdl_allow_next();
     const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
     const int h = blockIdx.x * kSplitSites + lane;
     const bool act = h < a.g.Vh;

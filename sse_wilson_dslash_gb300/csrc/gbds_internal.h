@@ -103,12 +103,16 @@ cudaError_t launch_dslash_xpay_df(const Geom &g, int recon, const void *gauge, c
 cudaError_t launch_f64_to_df(const void *in, void *out, size_t n, cudaStream_t stream);
 
 // site0: first caller site held by the packed buffer (0 for a full lattice).
-// df (prec 64): the internal field is double-float (dfloat.cuh).
+// df (prec 64): the internal field is double-float (dfloat.cuh).  chained: the
+// unpacking blocks may come up while the launch before still runs.  It saves
+// 3 us of a launch-bound call (8^4 FP32 on host arrays 32.3 -> 29.6), but the
+// early blocks' shared memory comes out of the running operator's L1 cache
+// (operator and unpack, double-float at 12^2x16x20: 23.2 us without, 38.3 with).
 cudaError_t launch_pack_spinor(const Geom &g, int prec, const void *psi_packed, const int *site_table,
                                int site0, int parity, void *spinor, cudaStream_t stream, bool df = false);
 cudaError_t launch_unpack_spinor(const Geom &g, int prec, const void *spinor, const int *site_table,
                                  int site0, int parity, void *psi_packed, cudaStream_t stream, bool df = false,
-                                 const SiteRange &range = {});
+                                 const SiteRange &range = {}, bool chained = false);
 cudaError_t launch_pack_gauge(const Geom &g, int prec, int recon, const void *u_packed,
                               const int *site_table, void *gauge, cudaStream_t stream);
 // Canonical order, in one launch: the links of the sites `range` of both

@@ -269,7 +269,7 @@ cudaError_t launch_pack_spinor(const Geom &g, int prec, const void *psi_packed, 
 
 cudaError_t launch_unpack_spinor(const Geom &g, int prec, const void *spinor, const int *site_table,
                                  int site0, int parity, void *psi_packed, cudaStream_t stream, bool df,
-                                 const SiteRange &range) {
+                                 const SiteRange &range, bool chained) {
     const int units = prec == 32 ? 6 : 12;
     df = df && prec == 64;
     const uint4 *src = static_cast<const uint4 *>(spinor);
@@ -277,9 +277,9 @@ cudaError_t launch_unpack_spinor(const Geom &g, int prec, const void *spinor, co
         uint4 *dst = static_cast<uint4 *>(psi_packed) + (size_t)(parity * g.Vh - site0) * units;
         const int first = range.first, end = range.end(g);
         const dim3 nb(blocks_for(end - first, kSpinorTile));
-        if (prec == 32) launch_pdl(unpack_spinor_tile<6>, nb, 128, stream, src, first, end, g.stride, dst);
-        else if (df) launch_pdl(unpack_spinor_tile<12, true>, nb, 128, stream, src, first, end, g.stride, dst);
-        else launch_pdl(unpack_spinor_tile<12>, nb, 128, stream, src, first, end, g.stride, dst);
+        auto k = prec == 32 ? unpack_spinor_tile<6> : df ? unpack_spinor_tile<12, true> : unpack_spinor_tile<12>;
+        if (chained) launch_pdl(k, nb, 128, stream, src, first, end, g.stride, dst);
+        else k<<<nb, 128, 0, stream>>>(src, first, end, g.stride, dst);
         count_launch();
         return cudaGetLastError();
     }
