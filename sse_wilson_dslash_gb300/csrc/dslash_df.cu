@@ -223,12 +223,9 @@ cudaError_t launch_dslash_df(const Geom &g, int recon, const void *gauge, const 
     return launch_dslash_t<dfloat>(g, recon, gauge, psi, res, isign, cb, block, variant, stream);
 }
 
-cudaError_t launch_dslash_xpay_df(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
-                                  double coef, void *res, double *partials, int isign, int cb, cudaStream_t stream) {
-    if (recon == 18 && !partials)
-        return launch_df3<true>(df_args(g, recon, gauge, psi, res, cb), isign, static_cast<const float4 *>(x),
-                                to_df(coef), stream);
-    return launch_dslash_xpay_t<dfloat>(g, recon, gauge, psi, x, to_df(coef), res, partials, isign, cb, stream);
+cudaError_t launch_dslash_xpay_df(const Geom &g, const void *gauge, const void *psi, const void *x, double coef, void *res,
+                                  int isign, int cb, cudaStream_t stream) {
+    return launch_df3<true>(df_args(g, 18, gauge, psi, res, cb), isign, static_cast<const float4 *>(x), to_df(coef), stream);
 }
 
 cudaError_t launch_f64_to_df(const void *in, void *out, size_t n, cudaStream_t stream) {

@@ -7,7 +7,7 @@
 // make one multiply-add of two 59-bit fixed-point numbers, with exact sums.
 // Here only the projection (96 additions a site) and the final conversion
 // (48) stay in FP64; the colour multiply and the accumulation run on
-// integers: 24^3x48 0.181 ms, 32^3x64 0.555 ms.  Bound by integer issue (ALU
+// integers: 24^3x48 0.175 ms, 32^3x64 0.541 ms (12-real links 0.301, 0.94).  Bound by integer issue (ALU
 // 55 %, IMAD pipe 47 %, FP64 pipe 42 % busy, 464 instructions a hop and
 // thread).
 //

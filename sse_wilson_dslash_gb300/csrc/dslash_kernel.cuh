@@ -579,11 +579,6 @@ __device__ __forceinline__ void sum_here(const double *partials, const SumHere &
     if (t == 0) sum_step(to.sc, to.mode, buf[0]);
 }
 
-// double-float: the per-thread sum goes in as one double
-__device__ __forceinline__ void block_sum_to(double *partials, dfloat v) {
-    block_sum_to<double>(partials, (double)v.hi + (double)v.lo);
-}
-
 // UPD: the CG's update in place of the store, r -= alpha (x + coef Dslash(psi))
 // with |r|^2 in the partials; nothing else is written.  A p is then neither
 // stored nor read back and the separate update pass is gone (x += alpha p moves
@@ -643,8 +638,7 @@ __global__ void __launch_bounds__(Bounds<MINB>::threads, Bounds<MINB>::blocks)
         else Field<T>::store_spinor(a.res, a.g.stride, h, acc);
     }
     if (partials) {
-        if constexpr (std::is_same_v<T, dfloat>) block_sum_to(partials, nrm);
-        else block_sum_to<T>(partials, nrm);
+        block_sum_to<T>(partials, nrm);
         if constexpr (MINB == 0 && std::is_same_v<T, float>) {
             if (here.ticket) sum_here(partials, here);
         }
@@ -749,7 +743,6 @@ __global__ void __launch_bounds__(128, 6)
 
 template <typename T> struct XpayMinb;
 template <> struct XpayMinb<float> { static constexpr int r18 = 6, r12 = 6; };
-template <> struct XpayMinb<dfloat> { static constexpr int r18 = 4, r12 = 4; };
 
 // Grid blocks of an xpay launch (the size `partials` must have).
 inline int xpay_blocks(const Geom &g) { return (g.Vh + 127) / 128; }

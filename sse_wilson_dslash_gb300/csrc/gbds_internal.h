@@ -97,8 +97,9 @@ cudaError_t launch_dslash_xpay_f64(const Geom &g, const void *gauge, const void 
 int dslash_variants_df();
 cudaError_t launch_dslash_df(const Geom &g, int recon, const void *gauge, const void *psi, void *res, int isign,
                              int cb, int block, int variant, cudaStream_t stream);
-cudaError_t launch_dslash_xpay_df(const Geom &g, int recon, const void *gauge, const void *psi, const void *x,
-                                  double coef, void *res, double *partials, int isign, int cb, cudaStream_t stream);
+// (18-real links)
+cudaError_t launch_dslash_xpay_df(const Geom &g, const void *gauge, const void *psi, const void *x, double coef, void *res,
+                                  int isign, int cb, cudaStream_t stream);
 // n complex elements FP64 -> double-float; in place allowed
 cudaError_t launch_f64_to_df(const void *in, void *out, size_t n, cudaStream_t stream);
 

@@ -416,7 +416,7 @@ cudaError_t apply_M_df(gbds_solver s, const void *in64, void *out_df, int isign,
     cudaError_t e = launch_f64_to_df(in64, s->xdf, spinor_bytes(g, 64) / 16, st);
     if (e == cudaSuccess) e = launch_dslash_df(g, 18, s->gauge_df, s->xdf, s->t64, isign, 0, 128, kDfVariant, st);
     if (e != cudaSuccess) return e;
-    return launch_dslash_xpay_df(g, 18, s->gauge_df, s->t64, s->xdf, -k2, out_df, nullptr, isign, 1, st);
+    return launch_dslash_xpay_df(g, s->gauge_df, s->t64, s->xdf, -k2, out_df, isign, 1, st);
 }
 
 // Fields within FP32's exponent range (the double-float operator's): |b|^2
