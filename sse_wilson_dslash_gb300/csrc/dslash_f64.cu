@@ -7,9 +7,9 @@
 // make one multiply-add of two 59-bit fixed-point numbers, with exact sums.
 // Here only the projection (96 additions a site) and the final conversion
 // (48) stay in FP64; the colour multiply and the accumulation run on
-// integers: 24^3x48 0.175 ms, 32^3x64 0.541 ms (12-real links 0.301, 0.94).  Bound by integer issue (ALU
-// 55 %, IMAD pipe 47 %, FP64 pipe 42 % busy, 464 instructions a hop and
-// thread).
+// integers: 24^3x48 0.175 ms, 32^3x64 0.533 ms (12-real links 0.301, 0.950).
+// Bound by integer issue (ALU 56 %, IMAD pipe 49 %, FP64 pipe 45 % busy, 464
+// instructions a hop and thread).
 //
 // Error against 64 bits (random SU(3), N(0,1) spinors): 1.45e-16 of the
 // result's norm, where the FP64 kernel had 1.96e-16 (it rounds each of the 6
