@@ -648,8 +648,7 @@ __device__ __forceinline__ float2 (*staged_links())[8][9] {
 // L1 data pipe 76 %, FMA pipe 42 %), so registers are capped for 28 warps:
 // 24^3x48, 16 rhs, FP32 0.320 -> 0.308 ms, FP32 pairs 0.308 -> 0.297 (prefetching
 // the next hop into registers at 12 or 16 warps: 0.340-0.391), BF16 8 rhs 0.150
-// -> 0.138; half + norm with a compile-time count keeps 20 warps (8 rhs 0.153
-// against 0.166).
+// -> 0.138; half + norm with a compile-time count keeps 20 warps.
 template <int FMT, int RECON, int ISIGN, int NRHS, int EPI>
 __global__ void __launch_bounds__(128, FMT == kFmtF16N && NRHS ? 5 : 7) dslash_gen3_kernel(const GenArgs a) {
     static_assert(NRHS == 0 ? EPI == 0 : NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides, or any count");
