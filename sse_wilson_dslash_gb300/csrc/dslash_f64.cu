@@ -7,7 +7,7 @@
 // make one multiply-add of two 59-bit fixed-point numbers, with exact sums.
 // Here only the projection (96 additions a site) and the final conversion
 // (48) stay in FP64; the colour multiply and the accumulation run on
-// integers: 24^3x48 0.175 ms, 32^3x64 0.533 ms (12-real links 0.301, 0.950).
+// integers: 24^3x48 0.179 ms, 32^3x64 0.552 ms (24^3x48 with 12-real links 0.299).
 // Bound by integer issue (ALU 56 %, IMAD pipe 49 %, FP64 pipe 45 % busy, 464
 // instructions a hop and thread).
 //
@@ -28,11 +28,18 @@
 // prefetching the next hop's spinors 0.189 ms).
 //
 // The scale of the sums follows the largest product so far (spinor exponent
-// + link exponent); when it grows, the sums are shifted.  An output is within
-// a few units of 2^-54 of the largest product of its colour, before its own
-// rounding.  Operands beyond the exponents the integers cover (2^177 and up,
-// infinities, NaN, or every product below 2^-646) take the plain FP64 path
-// at the end of the kernel, site by site.
+// + link exponent); when it grows, the sums are shifted.  So their error, a few
+// units of 2^-54 of the largest product of the colour, is absolute, and an output
+// whose own terms are all small beside it (a small spin, the smaller of the real
+// and imaginary part) would keep fewer bits than in FP64 arithmetic.  The moduli
+// of the hops' sums are therefore added up for each output (12 instructions a
+// hop, 24^3x48 174.7 -> 179.3 us), and the outputs that stay below half of the scale
+// (fix_resolved), with operands beyond the exponents the integers cover all of them
+// (2^177 and up, infinities, NaN, or every product below 2^-646), are formed in FP64
+// at the end of the kernel, site by site, from the half spinors that they take.
+// us at 24^3x48, against the kernel in FP64 arithmetic's 493 whatever the field:
+// random fields 179, unit links 184, one spin 2^-3 of the others 290, 2^-20 491; a
+// source of one spin 258, of one spin and colour 293, zero 234.
 #include "dslash_kernel.cuh"
 #include "fixpoint.cuh"
 
@@ -101,21 +108,24 @@ __device__ __forceinline__ void fx_sync(int grp) {
     else asm volatile("bar.sync %0, 96;" ::"r"(grp + 1) : "memory");
 }
 
-// acc += code * w for one complex, code 0: +1, 1: -1, 2: +i, 3: -i
+// acc += code * w for one complex, code 0: +1, 1: -1, 2: +i, 3: -i; m: the
+// moduli's high words of w, added up in seen
 template <int CODE>
-__device__ __forceinline__ void fx_acc(int64_t (&acc)[2], const int64_t (&w)[2]) {
+__device__ __forceinline__ void fx_acc(int64_t (&acc)[2], uint32_t (&seen)[2], const int64_t (&w)[2], const uint32_t (&m)[2]) {
     if constexpr (CODE == 0) { acc[0] += w[0]; acc[1] += w[1]; }
     else if constexpr (CODE == 1) { acc[0] -= w[0]; acc[1] -= w[1]; }
     else if constexpr (CODE == 2) { acc[0] -= w[1]; acc[1] += w[0]; }
     else { acc[0] += w[1]; acc[1] -= w[0]; }
+    seen[0] += m[CODE >> 1];
+    seen[1] += m[1 - (CODE >> 1)];
 }
 
 // What a thread (colour c of one site) keeps over its hops.
 struct FxSum {
-    int64_t acc[4][2];  // the four output spins, in units of 2^(e - 2 * 1023 - kFixUnit)
-    uint32_t e;         // the two operands' biased exponents at the scale of the sums
-    uint32_t top;       // the largest biased exponent of any operand
-    uint32_t any;       // the spinor exponents, or-ed: 0 when every source is 0 (or subnormal)
+    int64_t acc[4][2];    // the four output spins, in units of 2^(e - 2 * 1023 - kFixUnit)
+    uint32_t seen[4][2];  // the hops' moduli (fix_resolved)
+    uint32_t e;           // the two operands' biased exponents at the scale of the sums
+    uint32_t top;         // the largest biased exponent of any operand
 };
 
 // The thread's place: colour c, lane, group grp; act: it has a site.
@@ -166,7 +176,6 @@ __device__ __forceinline__ void fx_hop(const DslashArgs<double> &a, const FxThre
         eh[j] = sm.e[grp][buf][j][lane];
         const uint32_t eu = max(ex[j][0], ex[j][1]);
         S.top = max(S.top, max(eu, eh[j]));
-        S.any |= eh[j];
         et = max(et, eu + eh[j]);
     }
     if (et > S.e) {
@@ -174,92 +183,127 @@ __device__ __forceinline__ void fx_hop(const DslashArgs<double> &a, const FxThre
 #pragma unroll
         for (int sp = 0; sp < 4; sp++)
 #pragma unroll
-            for (int p = 0; p < 2; p++) S.acc[sp][p] = fix_sar(S.acc[sp][p], d);
+            for (int p = 0; p < 2; p++) {
+                S.acc[sp][p] = fix_sar(S.acc[sp][p], d);
+                S.seen[sp][p] = fix_shr(S.seen[sp][p], d);
+            }
         S.e = et;
     }
-    // W: the products' high parts; X: their cross parts, in units of 2^-32
-    // (the constant rounds them to nearest)
     int64_t W[2][2], X[2][2];
 #pragma unroll
     for (int k = 0; k < 2; k++)
 #pragma unroll
         for (int p = 0; p < 2; p++) {
             W[k][p] = 0;
-            X[k][p] = 1ll << 31;
+            X[k][p] = kFixHalf;
         }
 #pragma unroll
     for (int j = 0; j < 3; j++) {
         const uint32_t t0 = S.e - eh[j] + 3;
         const fix2 ur = to_fix(ud[j].x, t0 - ex[j][0]), ui = to_fix(ud[j].y, t0 - ex[j][1]);
-        const fix2 um = {-ui.n, ~ui.g};
-        // re += ur hr - ui hi, im += ur hi + ui hr (U^+: ui changes sign)
-        const fix2 a1 = DAG ? ui : um, a2 = DAG ? um : ui;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             const int4 q = sm.h[grp][buf][k][j][lane];
-            fix_mad(W[k][0], ur.n, q.x); fix_mad(X[k][0], ur.n, q.y); fix_mad(X[k][0], ur.g, q.x);
-            fix_mad(W[k][0], a1.n, q.z); fix_mad(X[k][0], a1.n, q.w); fix_mad(X[k][0], a1.g, q.z);
-            fix_mad(W[k][1], ur.n, q.z); fix_mad(X[k][1], ur.n, q.w); fix_mad(X[k][1], ur.g, q.z);
-            fix_mad(W[k][1], a2.n, q.x); fix_mad(X[k][1], a2.n, q.y); fix_mad(X[k][1], a2.g, q.x);
+            fix_cmad<DAG>(W[k], X[k], ur, ui, {q.x, q.y}, {q.z, q.w});
         }
     }
+    uint32_t m[2][2];
 #pragma unroll
     for (int k = 0; k < 2; k++) {
 #pragma unroll
-        for (int p = 0; p < 2; p++) W[k][p] += X[k][p] >> 32;
-        fx_acc<0>(S.acc[k], W[k]);
+        for (int p = 0; p < 2; p++) {
+            W[k][p] += X[k][p] >> 32;
+            m[k][p] = fix_modulus_hi(W[k][p]);
+        }
+        fx_acc<0>(S.acc[k], S.seen[k], W[k], m[k]);
     }
-    fx_acc<P::b2 ^ f>(S.acc[2], W[P::k2]);
-    fx_acc<P::b3 ^ f>(S.acc[3], W[P::k3]);
+    fx_acc<P::b2 ^ f>(S.acc[2], S.seen[2], W[P::k2], m[P::k2]);
+    fx_acc<P::b3 ^ f>(S.acc[3], S.seen[3], W[P::k3], m[P::k3]);
 }
 
-// Colour c of one hop in plain FP64.
-template <int MU, int SIGMA, bool DAG, int ND, int RECON>
-__device__ __forceinline__ void fx_plain_hop(const DslashArgs<double> &a, int c, int nbr, int hl, int lp,
-                                             cx<double> (&acc)[4]) {
-    using P = Proj<MU>;
-    constexpr int f = SIGMA > 0 ? 0 : 1;
-    const int stride = a.g.stride;
-    const double2 *U = reinterpret_cast<const double2 *>(a.gauge + (size_t)(lp * ND + MU) * a.link_block_bytes) + hl;
-    double2 u[3];
-    link_row<RECON, DAG>([&](int i) { return __ldg(U + (size_t)i * stride); }, c, u);
-    cx<double> w[2] = {};
+// Whether the real or the imaginary part is other than +-0.
+__device__ __forceinline__ bool nonzero(double2 v) {
+    return ((hi_word(v.x) | hi_word(v.y)) << 1 | (uint32_t)__double2loint(v.x) | (uint32_t)__double2loint(v.y)) != 0;
+}
+
+// Proj's coefficients of half spinor k by direction, two bits each; a lower
+// spin's is the conjugate of the one that the half spinor took that spin with.
+template <int K>
+constexpr uint32_t proj_codes() {
+    return K == 0 ? Proj<0>::a0 | Proj<1>::a0 << 2 | Proj<2>::a0 << 4 | Proj<3>::a0 << 6
+                  : Proj<0>::a1 | Proj<1>::a1 << 2 | Proj<2>::a1 << 4 | Proj<3>::a1 << 6;
+}
+
+// v with its sign bit changed by s (0 or 2^31)
+__device__ __forceinline__ double turn_sign(double v, uint32_t s) {
+    return __hiloint2double((int)(hi_word(v) ^ s), __double2loint(v));
+}
+
+// Half spinor K of one hop in FP64, colour c: w = (row c of U or U^+) h, added to
+// output spin K and to the lower spin of the pair where they are in `open`.  special: an operand is
+// infinite or NaN; else products with a factor 0 are left out (diluted sources,
+// sites without neighbours).
+template <int K, int RECON>
+__device__ __forceinline__ void fx_plain_half(const DslashArgs<double> &a, int c, int nbr, const double2 *U, bool dag, int mu,
+                                              int flip, uint32_t open, bool special, cx<double> (&p)[4]) {
+    const bool third = (mu < 2) == (K == 0);  // the lower spin is spin 3
+    const double2 *own = a.psi + (size_t)(K * 3) * a.g.stride + nbr, *low = a.psi + (size_t)(third ? 9 : 6) * a.g.stride + nbr;
+    double2 q[3], t[3];
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-        const cx<double> m = {u[j].x, DAG ? -u[j].y : u[j].y};
-        cx<double> s[4];
-#pragma unroll
-        for (int sp = 0; sp < 4; sp++) {
-            const double2 q = __ldg(a.psi + (size_t)(sp * 3 + j) * stride + nbr);
-            s[sp] = {q.x, q.y};
-        }
-        const cx<double> hs[2] = {cadd(s[0], mulc<P::a0 ^ f>(s[P::j0])), cadd(s[1], mulc<P::a1 ^ f>(s[P::j1]))};
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            w[k].r = fma(-m.i, hs[k].i, fma(m.r, hs[k].r, w[k].r));
-            w[k].i = fma(m.i, hs[k].r, fma(m.r, hs[k].i, w[k].i));
-        }
+        q[j] = __ldg(own + (size_t)j * a.g.stride);
+        t[j] = __ldg(low + (size_t)j * a.g.stride);
     }
-    acc[0] = cadd(acc[0], w[0]);
-    acc[1] = cadd(acc[1], w[1]);
-    acc[2] = cadd(acc[2], mulc<P::b2 ^ f>(w[P::k2]));
-    acc[3] = cadd(acc[3], mulc<P::b3 ^ f>(w[P::k3]));
+    bool used[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) used[j] = special || nonzero(q[j]) || nonzero(t[j]);
+    if (!(used[0] || used[1] || used[2])) return;
+    const auto ld = [&](int i) { return __ldg(U + (size_t)i * a.g.stride); };
+    double2 u[3];
+    if (dag) link_row<RECON, true>(ld, c, u);
+    else link_row<RECON, false>(ld, c, u);
+    const uint32_t code = (proj_codes<K>() >> (2 * mu) & 3) ^ flip;
+    const bool turned = code & 2;  // +-i
+    const uint32_t sx = (code ^ code >> 1) << 31, sy = code << 31;  // set for codes 1 and 2, 1 and 3
+    cx<double> w = {};
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        if (!used[j] || !(special || nonzero(u[j]))) continue;
+        const double hr = q[j].x + turn_sign(turned ? t[j].y : t[j].x, sx);
+        const double hi = q[j].y + turn_sign(turned ? t[j].x : t[j].y, sy);
+        const double mr = u[j].x, mi = dag ? -u[j].y : u[j].y;
+        w.r = fma(-mi, hi, fma(mr, hr, w.r));
+        w.i = fma(mi, hr, fma(mr, hi, w.i));
+    }
+    if (open & 3u << (2 * K)) p[K] = cadd(p[K], w);
+    if (!(open & (third ? 0xc0 : 0x30))) return;
+    // conj(code) w
+    const cx<double> l = turned ? cx<double>{turn_sign(w.i, ~sx & 1u << 31), turn_sign(w.r, ~sy & 1u << 31)}
+                                : cx<double>{turn_sign(w.r, sx), turn_sign(w.i, sy)};
+    if (third) p[3] = cadd(p[3], l);
+    else p[2] = cadd(p[2], l);
 }
 
-// whether every real of the site's source spinors is +-0
-template <int ND>
-__device__ __forceinline__ bool fx_sources_zero(const DslashArgs<double> &a, const Nbr &n) {
-    unsigned long long bits = 0;
-#pragma unroll
-    for (int mu = 0; mu < ND; mu++)
+// The outputs of colour c of which a part is marked in `open` (bit 2 s + part of
+// spin s), in FP64, from the half spinors that they take.
+template <int ND, int RECON, int ISIGN>
+__device__ __forceinline__ void fx_plain(const DslashArgs<double> &a, int c, int h, const Nbr &n, uint32_t open, bool special,
+                                         cx<double> (&p)[4]) {
 #pragma unroll 1
-        for (int i = 0; i < 12; i++) {
-            const double2 *p = a.psi + (size_t)i * a.g.stride;
-            const double2 f = __ldg(p + n.f[mu]), b = __ldg(p + n.b[mu]);
-            bits |= __double_as_longlong(f.x) | __double_as_longlong(f.y) | __double_as_longlong(b.x) |
-                    __double_as_longlong(b.y);
-        }
-    return (bits << 1) == 0;
+    for (int hop = 0; hop < 2 * ND; hop++) {
+        const int mu = hop >> 1;
+        const bool bwd = hop & 1;
+        // directions 0 and 1 pair spins 0, 3 and 1, 2; directions 2 and 3 spins 0, 2 and 1, 3
+        const uint32_t half0 = mu < 2 ? 0xc3 : 0x33;
+        const int f = mu == 0 ? n.f[0] : mu == 1 ? n.f[1] : mu == 2 ? n.f[2] : n.f[3];
+        const int b = mu == 0 ? n.b[0] : mu == 1 ? n.b[1] : mu == 2 ? n.b[2] : n.b[3];
+        const int nbr = bwd ? b : f, lp = bwd ? 1 - a.pt : a.pt;
+        const double2 *U =
+            reinterpret_cast<const double2 *>(a.gauge + (size_t)(lp * ND + mu) * a.link_block_bytes) + (bwd ? b : h);
+        const int flip = bwd == (ISIGN > 0) ? 1 : 0;
+        if (open & half0) fx_plain_half<0, RECON>(a, c, nbr, U, bwd, mu, flip, open, special, p);
+        if (open & ~half0) fx_plain_half<1, RECON>(a, c, nbr, U, bwd, mu, flip, open, special, p);
+    }
 }
 
 template <int ND, int RECON, int ISIGN, int MU, int GROUPS>
@@ -267,12 +311,6 @@ __device__ __forceinline__ void fx_dir(const DslashArgs<double> &a, const FxThre
                                        FxShared<GROUPS> &sm, FxSum &S) {
     fx_hop<MU, ISIGN, false, ND, RECON>(a, th, n.f[MU], h, a.pt, sm, S);
     fx_hop<MU, -ISIGN, true, ND, RECON>(a, th, n.b[MU], n.b[MU], 1 - a.pt, sm, S);
-}
-
-template <int ND, int RECON, int ISIGN, int MU>
-__device__ __forceinline__ void fx_plain_dir(const DslashArgs<double> &a, int c, int h, const Nbr &n, cx<double> (&acc)[4]) {
-    fx_plain_hop<MU, ISIGN, false, ND, RECON>(a, c, n.f[MU], h, a.pt, acc);
-    fx_plain_hop<MU, -ISIGN, true, ND, RECON>(a, c, n.b[MU], n.b[MU], 1 - a.pt, acc);
 }
 
 // res = Dslash psi, or (EPI 1) x + coef Dslash psi with partials[block] = the
@@ -298,8 +336,11 @@ __global__ void __launch_bounds__(96 * GROUPS, GROUPS == 1 ? 7 : 2)
     pdl_wait_prev();
     FxSum S;
 #pragma unroll
-    for (int s = 0; s < 4; s++) S.acc[s][0] = S.acc[s][1] = 0;
-    S.e = S.top = S.any = 0;
+    for (int s = 0; s < 4; s++) {
+        S.acc[s][0] = S.acc[s][1] = 0;
+        S.seen[s][0] = S.seen[s][1] = 0;
+    }
+    S.e = S.top = 0;
     fx_dir<ND, RECON, ISIGN, 0>(a, th, h, n, sm, S);
     fx_dir<ND, RECON, ISIGN, 1>(a, th, h, n, sm, S);
     fx_dir<ND, RECON, ISIGN, 2>(a, th, h, n, sm, S);
@@ -307,15 +348,25 @@ __global__ void __launch_bounds__(96 * GROUPS, GROUPS == 1 ? 7 : 2)
     double nrm = 0;
     if (th.act) {
         cx<double> r[4] = {};
+        uint32_t open = 0xff;  // outputs that the sums do not resolve: in FP64
         if (S.top <= kFxTop && S.e >= kFxLeast) {
+            open = 0;
             const double sc = __hiloint2double((int)((S.e - (2046 + kFixUnit - 1023)) << 20), 0);
 #pragma unroll
-            for (int sp = 0; sp < 4; sp++) r[sp] = {(double)S.acc[sp][0] * sc, (double)S.acc[sp][1] * sc};
-        } else if (S.any != 0 || S.top >= 2047 || !fx_sources_zero<ND>(a, n)) {
-            fx_plain_dir<ND, RECON, ISIGN, 0>(a, th.c, h, n, r);
-            fx_plain_dir<ND, RECON, ISIGN, 1>(a, th.c, h, n, r);
-            fx_plain_dir<ND, RECON, ISIGN, 2>(a, th.c, h, n, r);
-            if constexpr (ND == 4) fx_plain_dir<ND, RECON, ISIGN, 3>(a, th.c, h, n, r);
+            for (int sp = 0; sp < 4; sp++) {
+                r[sp] = {(double)S.acc[sp][0] * sc, (double)S.acc[sp][1] * sc};
+                open |= fix_resolved(S.seen[sp][0]) ? 0 : 1u << (2 * sp);
+                open |= fix_resolved(S.seen[sp][1]) ? 0 : 2u << (2 * sp);
+            }
+        }
+        if (open) {
+            cx<double> p[4] = {};
+            fx_plain<ND, RECON, ISIGN>(a, th.c, h, n, open, S.top >= 2047, p);
+#pragma unroll
+            for (int sp = 0; sp < 4; sp++) {
+                if (open >> (2 * sp) & 1) r[sp].r = p[sp].r;
+                if (open >> (2 * sp) & 2) r[sp].i = p[sp].i;
+            }
         }
 #pragma unroll
         for (int sp = 0; sp < 4; sp++) {
