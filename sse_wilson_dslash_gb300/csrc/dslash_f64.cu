@@ -58,9 +58,9 @@ struct FxShared {
 
 __device__ __forceinline__ double2 ld_link(const double2 *p, uint64_t pol) {
     double2 v;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-        : "=d"(v.x), "=d"(v.y)
-        : "l"(p), "l"(pol));
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"  // see ld_once
+                 : "=d"(v.x), "=d"(v.y)
+                 : "l"(p), "l"(pol));
     return v;
 }
 

@@ -150,7 +150,8 @@ template <typename T> struct Field;
 // The single right-hand-side operator reads every link once per
 // application: it loads them without allocating in L1 and marks their L2
 // lines first for eviction, so that L2 keeps the source spinors, which are
-// read by eight neighbours.
+// read by eight neighbours.  (volatile: a load stays behind pdl_wait_prev, also
+// volatile; the kernel that packs the links lets this one come up early.)
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t pol;
     asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
@@ -158,14 +159,16 @@ __device__ __forceinline__ uint64_t l2_evict_first_policy() {
 }
 __device__ __forceinline__ float2 ld_once(const float2 *p, uint64_t pol) {
     float2 v;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(pol));
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+                 : "=f"(v.x), "=f"(v.y)
+                 : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ float4 ld_once(const float4 *p, uint64_t pol) {
     float4 v;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-        : "l"(p), "l"(pol));
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p), "l"(pol));
     return v;
 }
 
