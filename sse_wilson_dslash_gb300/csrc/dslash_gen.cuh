@@ -212,6 +212,10 @@ struct RhsCgScalars {
     int pad;
 };
 
+// The register allocation of the kernels depends on this block's size: `reverse`
+// and `alpha` at its end (16 bytes more) changed the spills of half of the plain
+// kernels, FP32 with 4 rhs on 24^3x48 103.3 -> 104.3 us, FP32 pairs with one 42.6 ->
+// 44.0, half + norm with 2 66.3 -> 68.2.  So they sit in a gap and in a shared slot.
 struct GenArgs {
     Geom g;
     const char *psi;           // source checkerboard
@@ -224,15 +228,18 @@ struct GenArgs {
     // xpay epilogue: res = x + coef * D psi, |res|^2 partials
     const char *x;
     float coef;
+    int reverse;  // gen_block
     double *partials;
     // fused CG update (fully packed kernel, FP32 spin pairs): instead of
     // storing v = x + coef * D psi, r -= alpha_r v for active rhs, with
     // per-(block, rhs) |r|^2 partials
-    const RhsCgScalars *rsc;
+    union {
+        const RhsCgScalars *rsc;
+        const double *alpha;  // the same for nrhs 1 (16-bit storage, rvec an FP32 field)
+    };
     float4 *rvec;
-    int reverse;  // gen_block
-    const double *alpha;  // the same for nrhs 1 (16-bit storage, rvec an FP32 field)
 };
+static_assert(sizeof(GenArgs) == 128, "the kernels' register allocation was measured with this block");
 
 // NRHS > 0: compile-time count; NRHS == 0: a.nrhs at run time.
 template <int NRHS>
@@ -648,9 +655,13 @@ __device__ __forceinline__ float2 (*staged_links())[8][9] {
 // L1 data pipe 76 %, FMA pipe 42 %), so registers are capped for 28 warps:
 // 24^3x48, 16 rhs, FP32 0.320 -> 0.308 ms, FP32 pairs 0.308 -> 0.297 (prefetching
 // the next hop into registers at 12 or 16 warps: 0.340-0.391), BF16 8 rhs 0.150
-// -> 0.138; half + norm with a compile-time count keeps 20 warps.
+// -> 0.138; half + norm with a compile-time count takes 24 warps (8 rhs 152 us, 20
+// warps 162, 28 warps 167; 16 rhs 288, 291, 304), FP32 pairs with a run-time count 20
+// (9 rhs 213, 24 warps 215, 28 warps 220; 12 rhs 252, 253, 258; on 12^2x16x24 22.1,
+// 23.9, 24.2).
 template <int FMT, int RECON, int ISIGN, int NRHS, int EPI>
-__global__ void __launch_bounds__(128, FMT == kFmtF16N && NRHS ? 5 : 7) dslash_gen3_kernel(const GenArgs a) {
+__global__ void __launch_bounds__(128, FMT == kFmtF16N && NRHS ? 6 : FMT == kFmtF32Pairs && !NRHS ? 5 : 7)
+    dslash_gen3_kernel(const GenArgs a) {
     static_assert(NRHS == 0 ? EPI == 0 : NRHS >= 8 && NRHS <= 32, "8 to 32 right-hand sides, or any count");
     pdl_wait_prev();
     const int nr = nrhs_of<NRHS>(a);
