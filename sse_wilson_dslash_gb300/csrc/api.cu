@@ -122,28 +122,56 @@ extern "C" int gbds_op_create(gbds_op *op, const int dims[4], int nd, int prec, 
 // and for 16-bit storage the conversions, which the packed kernels write
 // straight into their pairs.  us at 24^3x48, 18-real links, plain kernel /
 // chosen one:
-//   FP32 (native)     4: 105 / 105   6: 149 / 149  12: 275 / 261
-//                    16: 360 / 284  24: 549 / 491  32: 721 / 568
-//   bfloat16          4:  91 /  91   6: 132 / 120  12: 250 / 198
-//                    16: 325 / 213  24: 485 / 358  32: 632 / 405
-//   half + norm       4: 123 /  96   6: 168 / 129  12: 316 / 223
-//                    16: 424 / 254  24: 603 / 415  32: 807 / 491
+//   FP32 (native)     4: 103 / 103   6: 149 / 149  12: 272 / 255
+//                    16: 360 / 282  24: 549 / 491  32: 721 / 571
+//   bfloat16          4:  89 /  89   6: 132 / 120  12: 248 / 195
+//                    16: 325 / 213  24: 485 / 358  32: 632 / 404
+//   half + norm       4: 119 /  95   6: 168 / 129  12: 317 / 220
+//                    16: 424 / 254  24: 603 / 415  32: 807 / 490
 // (odd counts: the two-rhs kernels do not apply; FP32 9: 216 / 217, bfloat16 7:
 // 151 with the plain kernel, 147 packed, half + norm 5: 144 / 121).  With 8 rhs
-// the default stays the plain kernel (half + norm: variant 2); gbds_op_autotune
-// or gbds_op_set_tuning reach the packed ones (FP32 193 / 166, bfloat16 172 / 133).
-// FP32 fields of few blocks (plain kernel: 128 pairs of a site and a rhs each)
-// take the plain kernel, whose blocks are shorter: 12 rhs on 12^2x16x24 (2592)
-// 20.8 / 23.9, on 16^3x20 (3840) 39.4 / 36.9; 10 rhs on 16^3x20 (3200) 30.9 /
-// 32.4, on 16^3x32 (5120) 50.8 / 49.6; 24 rhs on 10x14x12x20 (3150) 26.1 / 27.0, on
-// 12^2x16x24 (5184) 48.6 / 44.7.
-static int gen_variant(int nrhs, int format, int Vh) {
+// the default stays the plain kernel (half + norm: variant 2), as the interface's
+// tests fix it; gbds_op_autotune or gbds_op_set_tuning reach the packed ones (FP32
+// 189 / 165, bfloat16 169 / 132).
+//
+// Fields of few blocks (plain kernel: 128 pairs of a site and a rhs each) take
+// the plain kernel, whose blocks are shorter and which hides its loads while the
+// fields come out of L2.  us, plain / packed:
+//   FP32, from 9 rhs: 12 rhs on 12^2x16x24 (2592 blocks) 20.8 / 23.9, on 16^3x20
+//     (3840) 39.4 / 36.9; 10 rhs on 16^3x20 (3200) 30.9 / 32.4, on 16^3x32 (5120)
+//     50.8 / 49.6; 24 rhs on 10x14x12x20 (3150) 26.1 / 27.0, on 12^2x16x24 (5184)
+//     48.6 / 44.7.
+//   16-bit, two rhs a thread: by the pairs that the busiest of the 152 SMs gets, in
+//     CTAs of 128 / (nrhs / 2) sites against blocks of 128 pairs.  From 18 rhs always
+//     (18 rhs on 10^2x12x16, 1512 against 1382 pairs, half + norm 12.9 / 12.2, bfloat16 12.1 /
+//     10.6); 10 to 14 up to 1.13 times (half + norm 10 rhs on 12^2x16x24, 2000 against
+//     1920, 19.7 / 19.1, on 8^3x32, 750 against 640, 8.4 / 8.9; 12 rhs on 12^3x16 1.09:
+//     12.8 / 13.1, bfloat16 12.1 / 11.5); 6 rhs up to 1.03 times and above 600 plain
+//     blocks (12^2x16x24, 1260 against 1152, 12.9 / 14.3, bfloat16 12.1 / 13.0; 16^3x24,
+//     2016 against 2048, 21.4 / 20.6, 19.9 / 18.2; 8^3x24 5.0 / 5.3, 4.3 / 5.0).
+//   16-bit, one rhs a thread, from 9 rhs: half + norm 11 on 16^4 (2816) 24.7 / 26.2,
+//     9 on 16^3x24 (3456) 31.5 / 30.8.
+//   Half + norm, one rhs a thread, 4 to 7 rhs: by the fields' size, 18-real links:
+//     4 rhs on 16^3x32 (65 MB) 19.6 / 20.3, on 16^2x20x32 (81) 25.7 / 24.6; 5 rhs
+//     (72, 90) 24.2 / 26.3, 36.5 / 34.1; 7 rhs on 16^3x24 (64) 24.2 / 25.3, on
+//     16^3x32 (85) 36.2 / 34.2.  12-real: 5 rhs on 20^3x24 (87) 33.3 / 35.1, on
+//     20^2x24^2 (104) 41.9 / 41.9, 7 rhs on 20^3x24 (107) 47.6 / 46.3.
+static int gen_variant(int nrhs, int format, int recon, int Vh) {
     const bool bf16 = format == GBDS_SPINOR_BF16, half = bf16 || format == GBDS_SPINOR_F16_NORM;
+    const long long pairs = (long long)Vh * nrhs, blocks = pairs / 128;
     if (nrhs == 16 || nrhs == 32) return half ? 4 : 3;
     if (nrhs == 8) return format == GBDS_SPINOR_F16_NORM ? 2 : 0;
-    if (!half) return nrhs >= 8 && (long long)Vh * nrhs > 3500 * 128 ? 2 : 0;
-    if (nrhs % 2 == 0 && nrhs >= 6) return 3;
-    return nrhs >= (bf16 ? 9 : 4) ? 2 : 0;
+    if (!half) return nrhs >= 8 && pairs > 3500 * 128 ? 2 : 0;
+    if (nrhs % 2 == 0 && nrhs >= 6) {
+        const int sites = 128 / (nrhs / 2), ctas = (Vh + sites - 1) / sites;
+        const long long two = (ctas + 151) / 152 * (long long)sites * nrhs, plain = (pairs + 128 * 152 - 1) / (128 * 152) * 128;
+        if (nrhs >= 18) return 3;
+        return 100 * two <= (nrhs >= 10 ? 113 : blocks > 600 ? 103 : 0) * plain ? 3 : 0;
+    }
+    if (nrhs >= 9) return blocks > 2900 ? 2 : 0;
+    if (bf16 || nrhs < 4) return 0;
+    const long long bytes = 2 * pairs * gen_spinor_bytes(format) + 32LL * recon * Vh;  // two fields, all links
+    return bytes > (recon == 18 ? 73000000 : 92000000) ? 2 : 0;
 }
 
 extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int prec, int recon, int nrhs, int format) {
@@ -177,7 +205,7 @@ extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int pre
     // autotune chooses per shape.
     const bool gen = nrhs > 1 || (format != GBDS_SPINOR_NATIVE && format != GBDS_SPINOR_DOUBLE_FLOAT);
     o->block = 128;
-    o->variant = gen ? gen_variant(nrhs, format, g.Vh) : 0;
+    o->variant = gen ? gen_variant(nrhs, format, recon, g.Vh) : 0;
     if (!gen && prec == 32) f32_tuning(g, recon, &o->block, &o->variant);
     if (gen) o->g.zblock = gen_zblock(g, nrhs, format, recon);
     o->tensor_cores = 0;
