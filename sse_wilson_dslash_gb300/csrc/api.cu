@@ -371,6 +371,14 @@ std::mutex g_tune_mutex;
 std::map<std::array<int, 9>, std::array<int, 4>> g_tune_cache;
 }  // namespace
 
+// what gbds_op_dslash asks of its fields
+static int check_fields(const void *gauge, const void *psi, const void *res) {
+    if (!gauge || !psi || !res) return set_error(GBDS_ERROR_INVALID_VALUE, "NULL field pointer");
+    if (!aligned16(gauge) || !aligned16(psi) || !aligned16(res))
+        return set_error(GBDS_ERROR_INVALID_VALUE, "fields must be 16-byte aligned");
+    return GBDS_SUCCESS;
+}
+
 static bool tc_eligible(gbds_op op) {
     return (op->format == GBDS_SPINOR_BF16 || op->format == GBDS_SPINOR_F16_NORM) && (op->nrhs == 16 || op->nrhs == 32);
 }
@@ -384,7 +392,7 @@ extern "C" int gbds_op_autotune(gbds_op op, const void *gauge, const void *psi, 
     // the tensor-core kernel
     const bool v2ok = op->nrhs == 8 || op->nrhs == 16 || op->nrhs == 32;
     if (generic(op) && !tc_eligible(op) && !v2ok) return GBDS_SUCCESS;
-    if (op->prec == 64 && !double_float(op)) return GBDS_SUCCESS;  // FP64: one kernel and launch shape
+    if (op->prec == 64 && !double_float(op)) return check_fields(gauge, psi, res);  // FP64: one kernel and launch shape
     const std::array<int, 9> key = {op->g.L[0], op->g.L[1], op->g.L[2], op->g.L[3], op->g.nd,
                                     op->prec,   op->recon,  op->nrhs,   op->format};
     {
@@ -547,9 +555,8 @@ extern "C" int gbds_op_dslash(gbds_op op, const void *gauge, const void *psi, vo
     if (!op) return set_error(GBDS_ERROR_NOT_INITIALIZED, "op is NULL");
     if (isign != 1 && isign != -1) return GBDS_SUCCESS;  // reference: silent no-op
     if (cb != 0 && cb != 1) return set_error(GBDS_ERROR_INVALID_VALUE, "cb must be 0 or 1");
-    if (!gauge || !psi || !res) return set_error(GBDS_ERROR_INVALID_VALUE, "NULL field pointer");
-    if (!aligned16(gauge) || !aligned16(psi) || !aligned16(res))
-        return set_error(GBDS_ERROR_INVALID_VALUE, "fields must be 16-byte aligned");
+    const int rc = check_fields(gauge, psi, res);
+    if (rc != GBDS_SUCCESS) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (generic(op) && op->tensor_cores) {
         cudaError_t e = launch_gen_tc(op->format, op->g, op->recon, op->nrhs, gauge, psi, res, isign, cb, op->d_err, s);
