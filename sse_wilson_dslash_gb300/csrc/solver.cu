@@ -461,6 +461,18 @@ cudaError_t read_scalars(gbds_solver s, cudaStream_t st) {
     return e;
 }
 
+// A counter that is 0 for every stream, without the default stream: a caller may be
+// capturing a stream that synchronises with it, or have work on it to wait for.
+cudaError_t new_ticket(unsigned **ticket) {
+    cudaStream_t st = nullptr;
+    cudaError_t e = cudaMalloc(ticket, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(*ticket, 0, sizeof(unsigned), st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (st) cudaStreamDestroy(st);
+    return e;
+}
+
 // Record body(stream), which makes `launches` counted launches.  Where it cannot
 // be recorded, the graph stays empty and the iterations are launched one by one.
 template <typename BODY>
@@ -742,9 +754,7 @@ static int create_solver(gbds_solver *out, const int dims[4], const gbds_solver_
     const int parts = std::max(blocks(g), f32_partials(g, p->inner_recon));
     if (e == cudaSuccess) e = cudaMalloc(&s->partials, sizeof(double) * (size_t)parts);
     if (e == cudaSuccess) e = cudaMalloc(&s->sc, sizeof(Scalars));
-    if (e == cudaSuccess) e = cudaMalloc(&s->ticket, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(s->ticket, 0, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // zero for every stream
+    if (e == cudaSuccess) e = new_ticket(&s->ticket);
     if (e == cudaSuccess) e = cudaMallocHost(&s->hsc, sizeof(Scalars));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->read, cudaEventDisableTiming);
     if (e == cudaSuccess && p->inner_prec != 64 && single) record_inner(s);
@@ -1500,9 +1510,7 @@ extern "C" int gbds_bsolver_create(gbds_bsolver *out, const int dims[4], int nrh
     if (e == cudaSuccess && !fused_update(b)) e = cudaMalloc(&b->Ap, f32m);  // else never stored
     if (e == cudaSuccess) e = cudaMalloc(&b->bpartials, sizeof(double) * (size_t)bblocks(b) * nrhs);
     if (e == cudaSuccess) e = cudaMalloc(&b->bpartials2, sizeof(double) * (size_t)bblocks2(b) * nrhs);
-    if (e == cudaSuccess) e = cudaMalloc(&b->ticket, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(b->ticket, 0, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // zero for every stream
+    if (e == cudaSuccess) e = new_ticket(&b->ticket);
     if (e == cudaSuccess) e = cudaMalloc(&b->bsc, sizeof(BScalars) * nrhs);
     if (e == cudaSuccess) e = cudaMallocHost(&b->hbsc, sizeof(BScalars) * nrhs);
     if (e == cudaSuccess) e = cudaMalloc(&b->osc, sizeof(Scalars) * nrhs);
