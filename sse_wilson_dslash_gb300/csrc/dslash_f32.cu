@@ -90,8 +90,11 @@ cudaError_t launch_dslash_f32(const Geom &g, int recon, const void *gauge, const
     return launch_dslash_t<float>(g, recon, gauge, psi, res, isign, cb, block, variant, stream);
 }
 int dslash_variants(int prec) { return prec == 32 ? Variants<float>::n + 1 : 3; }
-// The launches with an epilogue follow f32_tuning's first two lines (small
-// lattices), else registers capped for 6 CTAs per SM.
+// The launches with an epilogue take four warps a site or uncapped registers where
+// f32_tuning does (there 64-thread blocks; here 128, a partial each), else registers
+// capped for 6 CTAs per SM.  Uncapped with 12-real links and 1065 to 1824 CTAs, us an
+// iteration of the FP32-inner solve, against the cap: 20^3x36 (1125) 104 / 108, 24^4
+// (1296) 110 / 115, 16^2x32x44 (1408) 124 / 125, 24^3x32 (1728) 141 / 141.
 namespace {
 
 template <bool UPD>
