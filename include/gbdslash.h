@@ -174,18 +174,20 @@ int gbds_op_dslash(gbds_op op, const void *gauge, const void *psi, void *res,
 /* Launch tuning of gbds_op_dslash: threads per block (0 = default 128; a
  * multiple of 32 up to 256) and a kernel variant.  Single rhs: 0 = registers
  * uncapped; 1.. = variants that cap registers for more resident warps, which
- * launch 128-thread blocks, and in FP32 the last one four warps a site; FP64 (native): every variant and block size is
- * accepted and runs the one kernel.  Several rhs or 16-bit storage: 0 = the plain
+ * launch 128-thread blocks, and in FP32 the last one four warps a site; FP64
+ * (native): every variant and block size is accepted and runs the one kernel.
+ * Several rhs or 16-bit storage: 0 = the plain
  * multi-RHS kernel, 1 = the packed FP32x2 form (8, 16, 32 rhs; the block
  * size is fixed at 128), 2 = projection, multiply and reconstruction all in
- * packed FP32x2 (2 rhs and more; 128-thread blocks; every storage format),
- * 3 = variant 2 with two rhs per thread, which share each staged link (FP32: 8,
+ * packed FP32x2, one rhs a thread (2 rhs and more; 128-thread blocks; every
+ * storage format; half + norm with 8 rhs in fields aligned to 32 bytes runs
+ * variant 3), 3 = variant 2 with two rhs per thread, which share each staged link (FP32: 8,
  * 16, 32 rhs; 16-bit formats: any even count from 4, other than 8, 16, 32 with
  * fields aligned to 32 bytes), and for the 16-bit formats 4 = variant 3 with
  * each thread's neighbour spinors prefetched two hops ahead by cp.async into
  * shared memory (8, 16, 32 rhs).  Where variant 4 does not apply, variant 3
  * runs, else variant 2, else the plain kernel (1 rhs, or variant 1 with another
- * count).  The default follows the count and the format.
+ * count).  The default follows the count, the format and the lattice's size.
  * gbds_op_num_variants gives the count.  Used by the autotuner. */
 int gbds_op_set_tuning(gbds_op op, int threads, int variant);
 int gbds_op_get_tuning(gbds_op op, int *threads, int *variant);
@@ -211,13 +213,14 @@ int gbds_op_get_site_order(gbds_op op, int *zblock);
  * for the same shape takes the cached choice without timing.  Operators with
  * several right-hand sides (or 16-bit storage) have these candidates: 0 the
  * plain multi-RHS kernel, 1 the colour multiply in packed FP32x2 arithmetic
- * on links staged per CTA (8, 16 or 32 rhs), 2 the whole hop in packed
- * FP32x2 (8, 16, 32 rhs), 3 the same with two rhs per thread, for the 16-bit
- * formats 4 (3 with cp.async prefetching)
+ * on links staged per CTA, 2 the whole hop in packed FP32x2, 3 the same with
+ * two rhs per thread, for the 16-bit formats 4 (3 with cp.async prefetching)
  * and, for 16-bit formats with 16 or 32 rhs, the tensor-core kernel
  * (gbds_op_set_tensor_cores); for a CUDA-core pick it then times the site
  * order (gbds_op_set_site_order): the natural order and z slabs of Lz/8
- * planes and up.  Synchronises `stream`. */
+ * planes and up.  Synchronises `stream`.  Nothing is timed, and the defaults
+ * stay, with counts of rhs other than 8, 16 and 32 and for FP64 (native), which
+ * has one launch shape. */
 int gbds_op_autotune(gbds_op op, const void *gauge, const void *psi, void *res, void *stream);
 
 /* Number of kernels this library has launched in this process (all kinds). */

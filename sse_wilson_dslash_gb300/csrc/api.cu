@@ -130,8 +130,8 @@ extern "C" int gbds_op_create(gbds_op *op, const int dims[4], int nd, int prec, 
 //                    16: 424 / 254  24: 603 / 415  32: 807 / 490
 // (odd counts: the two-rhs kernels do not apply; FP32 9: 216 / 217, bfloat16 7:
 // 151 with the plain kernel, 147 packed, half + norm 5: 144 / 121).  With 8 rhs
-// the default stays the plain kernel (half + norm: variant 2), as the interface's
-// tests fix it; gbds_op_autotune or gbds_op_set_tuning reach the packed ones (FP32
+// the default stays the plain kernel (half + norm: variant 2), the number that
+// tests/test_abi.py holds it to; gbds_op_autotune or gbds_op_set_tuning reach the packed ones (FP32
 // 189 / 165, bfloat16 169 / 132).
 //
 // Fields of few blocks (plain kernel: 128 pairs of a site and a rhs each) take
@@ -199,8 +199,8 @@ extern "C" int gbds_op_create_ex(gbds_op *op, const int dims[4], int nd, int pre
     o->nrhs = nrhs;
     o->format = format;
     // Single rhs, FP32: by the lattice (gbds_op_autotune refines it; FP64 has
-    // one launch shape).  Several rhs or another format: variant 0 = the plain multi-RHS kernel, 1 = its packed
-    // FP32x2 colour multiply, 2 = the whole hop packed, 3 = the same with two
+    // one launch shape).  Several rhs or another format: variant 0 = the plain
+    // multi-RHS kernel, 1 = its packed FP32x2 colour multiply, 2 = the whole hop packed, 3 = the same with two
     // rhs a thread, 4 = 3 with cp.async prefetching (16-bit storage);
     // autotune chooses per shape.
     const bool gen = nrhs > 1 || (format != GBDS_SPINOR_NATIVE && format != GBDS_SPINOR_DOUBLE_FLOAT);
@@ -385,11 +385,10 @@ static bool tc_eligible(gbds_op op) {
 
 extern "C" int gbds_op_autotune(gbds_op op, const void *gauge, const void *psi, void *res, void *stream) {
     if (!op) return set_error(GBDS_ERROR_NOT_INITIALIZED, "op is NULL");
-    // several right-hand sides: the candidates are the plain kernel, its
-    // packed FP32x2 form (8, 16, 32 rhs), for 16-bit and FP32-pair storage the
-    // fully packed kernel with one and with two rhs a thread, for 16-bit
-    // storage the latter with cp.async prefetching and, with 16 or 32 rhs,
-    // the tensor-core kernel
+    // 8, 16, 32 right-hand sides (other counts keep their default): the
+    // candidates are the plain kernel, its packed FP32x2 form, the fully packed
+    // kernel with one and with two rhs a thread, for 16-bit storage the latter
+    // with cp.async prefetching and, with 16 or 32 rhs, the tensor-core kernel
     const bool v2ok = op->nrhs == 8 || op->nrhs == 16 || op->nrhs == 32;
     if (generic(op) && !tc_eligible(op) && !v2ok) return GBDS_SUCCESS;
     if (op->prec == 64 && !double_float(op)) return check_fields(gauge, psi, res);  // FP64: one kernel and launch shape

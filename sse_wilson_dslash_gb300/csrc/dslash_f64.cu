@@ -8,7 +8,7 @@
 // Here only the projection (96 additions a site) and the final conversion
 // (48) stay in FP64; the colour multiply and the accumulation run on
 // integers: 24^3x48 0.179 ms, 32^3x64 0.552 ms (24^3x48 with 12-real links 0.299).
-// Bound by integer issue (ALU 56 %, IMAD pipe 49 %, FP64 pipe 45 % busy, 464
+// Bound by integer issue (ALU 57 %, IMAD pipe 49 %, FP64 pipe 44 % busy, 465
 // instructions a hop and thread).
 //
 // Error against 64 bits (random SU(3), N(0,1) spinors): 1.45e-16 of the

@@ -198,13 +198,14 @@ cudaError_t launch_gen_t(const Geom &g, int recon, int nrhs, const void *gauge, 
     // count from 4 (other than 16 and 32 with 256-bit loads, for fields aligned
     // to them), for FP32 8, 16 and 32; variant 4: for 16-bit storage and 8, 16, 32
     // rhs the same with cp.async prefetching; where these do not apply, variant 2
-    // (half + norm with 8 rhs takes the 256-bit loads under variant 2 as well: one
-    // rhs a thread 163 us at 24^3x48 and 36.0 at 16^3x32, two 149 and 32.9)
+    // (half + norm with 8 rhs takes the 256-bit loads under variant 2, its default,
+    // as well: one rhs a thread 152 us at 24^3x48 and 34.8 at 16^3x32, two 147 and
+    // 32.3)
     constexpr bool half = FMT == kFmtBF16 || FMT == kFmtF16N;
     const bool aligned32 = ((reinterpret_cast<uintptr_t>(psi) | reinterpret_cast<uintptr_t>(res)) & 31u) == 0;
     const bool v5 = variant == 4 && packed_nrhs && half && !epi;
-    const bool v4w = (variant == 3 || variant == 4 || (variant == 2 && FMT == kFmtF16N && nrhs == 8)) && half && nrhs >= 4 && nrhs % 2 == 0 && nrhs != 16 && nrhs != 32 &&
-                     aligned32 && !epi;
+    const bool v4w = (variant == 3 || variant == 4 || (variant == 2 && FMT == kFmtF16N && nrhs == 8)) && half &&
+                     nrhs >= 4 && nrhs % 2 == 0 && nrhs != 16 && nrhs != 32 && aligned32 && !epi;
     const bool v4 = (variant == 3 || variant == 4) && packed_nrhs && !epi;
 #define GBDS_GEN(R, S)                                                   \
     do {                                                                 \

@@ -124,14 +124,15 @@ cudaError_t launch_pack_fields(const Geom &g, int prec, int recon, const void *u
                                const SiteRange &range, const void *psi_packed, int parity, void *spinor,
                                cudaStream_t stream, bool chained = false);
 
-// Generalised Dslash (dslash_gen_*.cu): FP32 arithmetic and links, nrhs in
-// {1,2,4,8,16,32}, spinor formats 0 FP32, 1 BF16, 2 FP16 + norm, 3 FP32 in
+// Generalised Dslash (dslash_gen_*.cu): FP32 arithmetic and links, nrhs 1 to 32
+// (with an epilogue 1, 2, 4, 8, 16, 32), spinor formats 0 FP32, 1 BF16, 2 FP16 + norm, 3 FP32 in
 // spin pairs.  x != nullptr selects the xpay epilogue res = x + coef * D psi
 // with |res|^2 partials (one per 128-thread block for nrhs 1, one per block
 // and rhs otherwise).
 // variant 1: the colour multiply in packed FP32x2 arithmetic on links staged
-// per CTA (nrhs 8, 16, 32; other counts take variant 0).  variant 2 (formats
-// 1, 2, 3): the whole hop in packed FP32x2 (nrhs 8, 16, 32).
+// per CTA (nrhs 8, 16, 32; other counts take variant 0).  variant 2: the whole
+// hop in packed FP32x2 (nrhs from 2; with an epilogue format 3 and nrhs 8, 16, 32).
+// variants 3, 4: launch_gen_t.
 cudaError_t launch_gen_f32(const Geom &g, int recon, int nrhs, const void *gauge, const void *psi, void *res, int isign,
                            int cb, const void *x, float coef, double *partials, cudaStream_t st, int variant = 0);
 // reverse (FP32 pairs, packed kernels): the blocks go through the lattice from
