@@ -202,12 +202,16 @@ __device__ __forceinline__ void pack_gauge_block(const unsigned long long *packe
 
 // The first spinor_blocks blocks move a spinor, the others the links of sites
 // [first, end) of both checkerboards, ceil((end - first) / kGaugeTile) blocks each.
+// early: the launch behind it is one of a call on host arrays (more of these, or the
+// single-rhs operator, whose link loads stay behind the wait); what a caller
+// launches behind a packing call of its own comes up when this ends.
 template <typename T, int RECON>
 __global__ void __launch_bounds__(128) pack_fields_tile(const uint4 *psi, uint4 *__restrict__ soa, int spinor_blocks,
                                                          const unsigned long long *links, const Geom g,
-                                                         char *__restrict__ gauge, size_t block_bytes, int first, int end) {
+                                                         char *__restrict__ gauge, size_t block_bytes, int first, int end,
+                                                         int early) {
     extern __shared__ uint4 tile[];
-    pdl_allow_next();
+    if (early) pdl_allow_next();
     int b = blockIdx.x;
     if (b < spinor_blocks) {
         const int h0 = b * kSpinorTile;
@@ -228,10 +232,12 @@ void launch_pack_tile(const Geom &g, const uint4 *psi, uint4 *soa, const unsigne
     const int ns = psi ? (int)blocks_for(g.Vh, kSpinorTile) : 0;
     const unsigned nl = 2 * blocks_for(end - first, kGaugeTile);
     const size_t smem = (size_t)sizeof(T) * (ns ? kSpinorTile * 24 : kGaugeTile * 72);
+    const int early = ns || chained;
     if (chained)
-        launch_pdl_smem(pack_fields_tile<T, RECON>, dim3(ns + nl), 128, smem, st, psi, soa, ns, links, g, gauge, block_bytes, first, end);
+        launch_pdl_smem(pack_fields_tile<T, RECON>, dim3(ns + nl), 128, smem, st, psi, soa, ns, links, g, gauge, block_bytes,
+                        first, end, early);
     else
-        pack_fields_tile<T, RECON><<<ns + nl, 128, smem, st>>>(psi, soa, ns, links, g, gauge, block_bytes, first, end);
+        pack_fields_tile<T, RECON><<<ns + nl, 128, smem, st>>>(psi, soa, ns, links, g, gauge, block_bytes, first, end, early);
 }
 
 }  // namespace
