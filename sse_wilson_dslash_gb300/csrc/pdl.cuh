@@ -16,7 +16,9 @@ namespace gbds {
 // next grid is then launched, its parameters in place, when this one ends).  us
 // with the early start / without: FP64 on 12^2x16x20 22.5 / 16.6 (16^3x32, two
 // waves: 38.2 / 38.7); 12 rhs on 8^3x16 9.2 / 6.2; 2 rhs on 10x14x12x20 6.9 /
-// 5.3; FP32 on 32^3x40 78.2 / 79.6.
+// 5.3; FP32 on 32^3x40 78.2 / 79.6.  The multi-RHS kernels never allow it: on large
+// lattices it makes no difference (24^3x48: FP32 12 rhs 260.9 / 260.7, bfloat16 32
+// rhs 406.6 / 406.5), on 16^3x32 FP32 with 4 rhs takes 20.3 / 19.7.
 __device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_prev() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
